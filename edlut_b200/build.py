@@ -17,7 +17,12 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 OUT = os.path.join(OUT_DIR, "libedlut_b200.so")
-SOURCES = ["eb_kernels.cu", "eb_runtime.cu", "eb_record.cu", "eb_fold.cu", "eb_sweep.cu", "eb_adjoint.cu", "eb_tables.cpp", "eb_cfg.cpp"]
+# (source, defines): a file listed several times is compiled once per set of defines,
+# so that its template instantiations compile in parallel (the longest first)
+SOURCES = ([("eb_persist.cu", ("EB_CLASS=%d" % c,)) for c in (2, 1, 0)]
+           + [("eb_update.cu", ("EB_KIND=%d" % k, "EB_INTEG=%d" % i)) for k in (3, 2, 1) for i in (3, 2, 1, 0)]
+           + [(f, ()) for f in ("eb_kernels.cu", "eb_runtime.cu", "eb_record.cu", "eb_fold.cu", "eb_sweep.cu", "eb_adjoint.cu",
+                                "eb_tables.cpp", "eb_cfg.cpp")])
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -54,18 +59,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
     headers.append(os.path.join(ROOT, "include", "edlut_b200.h"))
     newest_header = max(os.path.getmtime(h) for h in headers)
 
-    def compile_one(src):
+    def compile_one(item):
+        src, defines = item
         path = os.path.join(CSRC, src)
-        obj = os.path.join(obj_dir, src + ".o")
+        obj = os.path.join(obj_dir, "".join([src, *("." + d.replace("=", "") for d in defines), ".o"]))
         if (not force and os.path.exists(obj)
                 and os.path.getmtime(obj) > max(os.path.getmtime(path), newest_header)):
             return obj, None
-        cmd = [nvcc(), *_compile_flags(), "-c", path, "-o", obj + ".tmp"]
+        cmd = [nvcc(), *_compile_flags(), *("-D" + d for d in defines), "-c", path, "-o", obj + ".tmp"]
         if verbose:
             print(" ".join(cmd))
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            return obj, "nvcc failed on %s:\n%s%s" % (src, r.stdout[-4000:], r.stderr[-4000:])
+            return obj, "nvcc failed on %s %s:\n%s%s" % (src, " ".join(defines), r.stdout[-4000:], r.stderr[-4000:])
         os.replace(obj + ".tmp", obj)
         return obj, None
 

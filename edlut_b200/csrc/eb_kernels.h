@@ -18,6 +18,9 @@ void launch_post_stdp(const PopDev &P, const NetDev &N, int rel, int max_chunks,
 // Deferred post-synaptic STDP: apply the spikes noted since the last flush to the
 // synapses of every neuron with more than keep of them (3 launches).
 void launch_flush_post(const PopDev &P, const NetDev &N, int max_chunks, uint32_t keep, int blocks, cudaStream_t st);
+// Weights of the synapses at target-major positions tpos[0..c) into / from w[0..c).
+void launch_weights_get(const SynRec *syn, const uint32_t *tpos, int64_t c, float *w, cudaStream_t st);
+void launch_weights_set(SynRec *syn, const uint32_t *tpos, int64_t c, const float *w, cudaStream_t st);
 void launch_advance(int64_t *step, int K, cudaStream_t st);
 
 constexpr int kMaxPersistPops = 16;

@@ -207,8 +207,6 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
         return tgt[a] < tgt[b];
     });
     if (out_sorted_perm) std::copy(ord.begin(), ord.end(), out_sorted_perm);
-    spos_of.assign(m, 0);
-    for (int64_t s = 0; s < m; ++s) spos_of[ord[s]] = s;
     std::vector<int64_t> out_ptr(n_neurons + 1, 0);
     for (int64_t k = 0; k < m; ++k) out_ptr[src[k] + 1]++;
     for (int64_t i = 0; i < n_neurons; ++i) out_ptr[i + 1] += out_ptr[i];
@@ -225,8 +223,8 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
         if (tgt[a] != tgt[b]) return tgt[a] < tgt[b];
         return (rule[a] >= 0) > (rule[b] >= 0);
     });
-    tpos_of.assign(m, 0);
-    for (int64_t t = 0; t < m; ++t) tpos_of[tord[t]] = t;
+    std::vector<uint32_t> tpos_of(m);
+    for (int64_t t = 0; t < m; ++t) tpos_of[tord[t]] = (uint32_t)t;
     for (int64_t i = 0; i < n_neurons; ++i) {
         int64_t e = in_ptr[i];
         while (e < in_ptr[i + 1] && rule[tord[e]] >= 0) ++e;
@@ -238,7 +236,7 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
     for (int64_t s = 0; s < m; ++s) {
         int64_t k = ord[s];
         h_out_tgt[s] = (uint32_t)tgt[k];
-        h_out_tpos[s] = (uint32_t)tpos_of[k];
+        h_out_tpos[s] = tpos_of[k];
         h_out_units[s] = (uint16_t)units[k];
     }
     std::vector<int64_t> grp_ptr(n_neurons + 1, 0);
@@ -316,6 +314,7 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
         }
         if ((rc = upload(this, &N.syn, hs))) return rc;
     }
+    if ((rc = upload(this, &d_tpos, tpos_of))) return rc;
     std::vector<float> rp;
     for (auto &r : rules) {
         rp.push_back(r[0]); rp.push_back(r[1]); rp.push_back(r[2]); rp.push_back(r[3]);
@@ -1525,32 +1524,38 @@ int eb_get_trace(eb_ctx *ctx, float *out) {
     return EB_OK;
 }
 
-int eb_get_weights(eb_ctx *ctx, float *w) {
+// Weights in network-file order between the host and the synapse records: the
+// device gathers (scatters) them, kWeightChunk at a time through one kept staging
+// buffer, so 4 bytes a synapse cross to the host instead of its 32-byte record and
+// the host permutes nothing.
+static int weights_io(eb_ctx *ctx, float *w, bool get) {
     if (!ctx || !w) { set_error("bad argument"); return EB_ERR_ARG; }
     if (!ctx->finalized) { set_error("not finalized"); return EB_ERR_STATE; }
+    CK(cudaSetDevice(ctx->device));
     int rc;
-    if ((rc = ctx->flush_post())) return rc;  // deferred post-synaptic updates first
-    CK(cudaStreamSynchronize(ctx->stream));
+    // deferred post-synaptic updates first: they belong to the weights read, or to the old ones
+    if ((rc = ctx->flush_post())) return rc;
     const int64_t m = (int64_t)ctx->src.size();
-    std::vector<SynRec> h(m);
-    if (m) CK(cudaMemcpy(h.data(), ctx->net.syn, sizeof(SynRec) * (size_t)m, cudaMemcpyDeviceToHost));
-    for (int64_t k = 0; k < m; ++k) w[k] = h[ctx->tpos_of[k]].w;
+    const int64_t chunk = std::min<int64_t>(m, kWeightChunk);
+    if (m && !ctx->d_wstage && (rc = ctx->dalloc((void **)&ctx->d_wstage, sizeof(float) * (size_t)chunk))) return rc;
+    for (int64_t k = 0; k < m; k += chunk) {
+        const int64_t c = std::min(chunk, m - k);
+        if (get) {
+            launch_weights_get(ctx->net.syn, ctx->d_tpos + k, c, ctx->d_wstage, ctx->stream);
+            CK(cudaMemcpyAsync(w + k, ctx->d_wstage, sizeof(float) * (size_t)c, cudaMemcpyDeviceToHost, ctx->stream));
+        } else {
+            CK(cudaMemcpyAsync(ctx->d_wstage, w + k, sizeof(float) * (size_t)c, cudaMemcpyHostToDevice, ctx->stream));
+            launch_weights_set(ctx->net.syn, ctx->d_tpos + k, c, ctx->d_wstage, ctx->stream);
+        }
+        CK(cudaGetLastError());
+        ctx->launches += 1;
+    }
+    CK(cudaStreamSynchronize(ctx->stream));
     return EB_OK;
 }
 
-int eb_set_weights(eb_ctx *ctx, const float *w) {
-    if (!ctx || !w) { set_error("bad argument"); return EB_ERR_ARG; }
-    if (!ctx->finalized) { set_error("not finalized"); return EB_ERR_STATE; }
-    const int64_t m = (int64_t)ctx->src.size();
-    std::vector<SynRec> h(m);
-    int rc;
-    if ((rc = ctx->flush_post())) return rc;  // pending post-synaptic updates belong to the old weights
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (m) CK(cudaMemcpy(h.data(), ctx->net.syn, sizeof(SynRec) * (size_t)m, cudaMemcpyDeviceToHost));
-    for (int64_t k = 0; k < m; ++k) h[ctx->tpos_of[k]].w = w[k];
-    if (m) CK(cudaMemcpy(ctx->net.syn, h.data(), sizeof(SynRec) * (size_t)m, cudaMemcpyHostToDevice));
-    return EB_OK;
-}
+int eb_get_weights(eb_ctx *ctx, float *w) { return weights_io(ctx, w, true); }
+int eb_set_weights(eb_ctx *ctx, const float *w) { return weights_io(ctx, const_cast<float *>(w), false); }
 
 int eb_set_random_seed(eb_ctx *ctx, uint32_t seed) {
     if (!ctx) { set_error("null context"); return EB_ERR_ARG; }

@@ -16,6 +16,9 @@ namespace eb {
 
 void set_error(const char *fmt, ...);
 
+// Weights that one staging pass of eb_get_weights / eb_set_weights moves (32 MB).
+constexpr int64_t kWeightChunk = 8 << 20;
+
 // Most steps one launch of a captured graph runs for one population.
 constexpr int kMaxFuse = 8;
 
@@ -66,7 +69,8 @@ struct eb_ctx {
     double dt_s = 0.0;
     int R = 0;
     std::vector<int> pop_of;
-    std::vector<int64_t> spos_of, tpos_of;
+    uint32_t *d_tpos = nullptr;   // file order -> target-major position of each synapse
+    float *d_wstage = nullptr;    // weights on their way to or from the host (first use)
     eb::NetDev net{};
     int64_t *d_step = nullptr;
     bool has_inputs = false;

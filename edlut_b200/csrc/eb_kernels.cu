@@ -1,6 +1,5 @@
 // Launchers of the step kernels, and the kernels that belong to no neuron model:
-// input fan-out, Poisson generators, eager post-synaptic STDP, the deferred-STDP
-// flush and the weight transfer.  The update kernels are in eb_step.cuh.
+// input fan-out, Poisson generators, the deferred-STDP flush and the weight transfer.  The update kernels are in eb_step.cuh.
 #include "eb_step.cuh"
 
 namespace eb {
@@ -13,8 +12,6 @@ namespace eb {
 // 32 bits, so 32-bit arithmetic gives the reference's sequence.
 __global__ void __launch_bounds__(256) k_update_poisson(PopDev P, NetDev N, int rel, int nsteps, double push_inv_dt) {
     const int64_t k0 = cur_step(N, rel);
-    const bool list = nsteps == 1;
-    if (list && blockIdx.x == 0 && threadIdx.x == 0) P.spk_count[(k0 + 1) & 1] = 0;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const double thr = i < P.n ? P.pthr[i] : 0.0;
     uint32_t x = i < P.n ? P.lcg[i] : 0u;
@@ -26,16 +23,10 @@ __global__ void __launch_bounds__(256) k_update_poisson(PopDev P, NetDev N, int 
             const float r = (float)x / (float)2147483647;
             sp = thr > (double)r;
         }
-        compact_spikes(P, N, k, i, sp, list);
+        compact_spikes(P, N, k, i, sp, false);
         if (push_inv_dt > 0.0) warp_push(P, N, k, i, sp, push_inv_dt);
     }
     if (i < P.n && thr > 0.0) P.lcg[i] = x;
-}
-
-__global__ void __launch_bounds__(256) k_push(PopDev P, NetDev N, int rel, double inv_dt) {
-    const int64_t k = cur_step(N, rel);
-    const uint32_t ns = min(P.spk_count[k & 1], (uint32_t)P.n);
-    for (int64_t s = blockIdx.x; s < ns; s += gridDim.x) push_spike(P, N, k, s, inv_dt);
 }
 
 // Input spikes of steps k .. k+nsteps-1.  Their deliveries are independent, so the
@@ -50,13 +41,6 @@ __global__ void __launch_bounds__(256) k_input_push(NetDev N, int rel, int nstep
         while (k + 1 < k0 + nsteps && N.in_start[k + 1] <= q) ++k;
         input_spike(N, k, q, inv_dt);
     }
-}
-
-__global__ void __launch_bounds__(256) k_post_stdp(PopDev P, NetDev N, int rel, int max_chunks) {
-    const int64_t k = cur_step(N, rel);
-    const uint32_t ns = min(P.spk_count[k & 1], (uint32_t)P.n);
-    const int64_t items = (int64_t)ns * max_chunks;
-    for (int64_t item = blockIdx.x; item < items; item += gridDim.x) post_item(P, N, k, item / max_chunks, item % max_chunks);
 }
 
 int persist_class_of(int kind, int integ) {
@@ -132,16 +116,8 @@ void launch_update(const PopDev &P, const NetDev &N, int rel, int nsteps, double
     }
 }
 
-void launch_push(const PopDev &P, const NetDev &N, int rel, double inv_dt, int blocks, int threads, cudaStream_t st) {
-    k_push<<<blocks, threads, 0, st>>>(P, N, rel, inv_dt);
-}
-
 void launch_input_push(const NetDev &N, int rel, int nsteps, double inv_dt, int blocks, int threads, cudaStream_t st) {
     k_input_push<<<blocks, threads, 0, st>>>(N, rel, nsteps, inv_dt);
-}
-
-void launch_post_stdp(const PopDev &P, const NetDev &N, int rel, int max_chunks, int blocks, cudaStream_t st) {
-    k_post_stdp<<<blocks, kPostThreads, 0, st>>>(P, N, rel, max_chunks);
 }
 
 // Bring every plastic synapse onto the population up to date with its target's

@@ -32,7 +32,6 @@ struct HostPop {
     bool output = true;         // spikes go to eb_write_spikes (the layer line's output column)
     bool monitor = false;       // states go to the state monitor file (the layer line's log column)
     int post_chunks = 1;
-    int push_threads = 32;
     std::vector<float> rates;   // Poisson generators: per-neuron frequency (Hz)
     PopDev dev{};
 };
@@ -92,7 +91,7 @@ struct eb_ctx {
     std::vector<std::vector<ChainDep>> chain_deps;
     std::vector<cudaEvent_t> chain_ev;         // [chain][step of the graph]
     bool chains_ok = false, chains_enabled = true;
-    int chain_fuse = 1;                        // steps per launch in a chain (a power of two)
+    int chain_fuse = 1;                        // steps per launch in a chain
     // time grid and inputs
     std::vector<double> t_host;
     double *d_tstep = nullptr;

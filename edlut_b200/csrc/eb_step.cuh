@@ -8,12 +8,10 @@
 //                  conductances in the reference's delivery order (arrival time,
 //                  then synapse order) with the STDP pre-synaptic update, advance
 //                  the neuron one integration step, test the spike condition,
-//                  compact the spiking neurons (warp ballot) and record them
-//   k_post_stdp    per population with plastic inputs: post-synaptic STDP update
-//                  of every plastic input synapse of each neuron that spiked
-//   k_push         per population with outputs: fan each spike out into the
-//                  arrival buckets of its targets (integer atomics only; the
-//                  fold sorts, so results do not depend on atomic order)
+//                  compact the spiking neurons (warp ballot), record them and fan
+//                  each spike out into the arrival buckets of its targets (integer
+//                  atomics only; the fold sorts, so results do not depend on atomic
+//                  order); post-synaptic STDP is deferred (apply_pending)
 // The step index is read from device memory (base + offset baked into the
 // launch), so one captured CUDA graph of K steps replays for any K steps.
 //
@@ -301,7 +299,7 @@ __device__ __forceinline__ void record_trace(const PopDev &P, const NetDev &N, i
 }
 
 // Warp-aggregated append of the spiking lanes to the population spike list (when
-// list is set: launches of one step, whose list the eager post-synaptic and
+// list is set: the persistent kernel, whose eager post-synaptic and
 // separate fan-out kernels read) and to the recording buffer.
 __device__ __forceinline__ void compact_spikes(const PopDev &P, const NetDev &N, int64_t k, int64_t i, bool sp,
                                                bool list = true) {
@@ -483,9 +481,7 @@ __device__ __forceinline__ void update_narrow_tile(const PopDev &P, const NetDev
     }
 }
 
-// Steps k .. k+nsteps-1 of one tile, the state in registers between them.  Only a
-// launch of one step keeps the population spike list (with several, no kernel
-// reads it: fan-out is done here and post-synaptic STDP is deferred).
+// Steps k .. k+nsteps-1 of one tile, the state in registers between them.
 // push_inv_dt > 0: also fan out the spikes (1 / step, for arrival_step).
 // HH under BDF holds the Newton state (Jacobian, inverse, history) in about 120
 // registers, which leaves 2 blocks per SM; bounded to 3 blocks (80 registers, a
@@ -502,8 +498,6 @@ template <int KIND, int INTEG, int EN, int MON>
 __global__ void __launch_bounds__(kNarrowTile, narrow_min_blocks(KIND, INTEG)) k_update_narrow(PopDev P, NetDev N, int rel, int nsteps,
                                                                 double push_inv_dt) {
     const int64_t k = cur_step(N, rel);
-    const bool list = nsteps == 1;
-    if (list && blockIdx.x == 0 && threadIdx.x == 0) P.spk_count[(k + 1) & 1] = 0;
     const int64_t i = (int64_t)blockIdx.x * kNarrowTile + threadIdx.x;
     const bool active = i < P.n;
     float x[kMaxVars];
@@ -512,7 +506,7 @@ __global__ void __launch_bounds__(kNarrowTile, narrow_min_blocks(KIND, INTEG)) k
         load_state<KIND>(P, i, x);
         ax = load_aux<KIND, INTEG>(P, i);
     }
-    for (int s = 0; s < nsteps; ++s) narrow_step<KIND, INTEG, EN, MON>(P, N, k + s, i, active, x, ax, list, push_inv_dt);
+    for (int s = 0; s < nsteps; ++s) narrow_step<KIND, INTEG, EN, MON>(P, N, k + s, i, active, x, ax, false, push_inv_dt);
     if (active) {
         store_state<KIND>(P, i, x);
         store_aux<KIND, INTEG>(P, i, ax);
@@ -939,10 +933,10 @@ __device__ __forceinline__ void ordered_sum(const WideSmem &S, uint32_t o0, uint
 
 // Lane 0 of warp 0, after step ks's conductances are in x: integrate, test the
 // spike, note it for deferred post-synaptic STDP (global ring and its staged
-// copy), trace, spike list and recording.  Returns the spike flag.
+// copy), trace and recording.  Returns the spike flag.
 template <int KIND, int INTEG, int MON = 2, int EN = -1>
 __device__ __forceinline__ int wide_advance(const PopDev &P, const NetDev &N, int64_t ks, int64_t i, WideSmem &S,
-                                            float *x, NeuronAux &ax, bool list, bool ring) {
+                                            float *x, NeuronAux &ax, bool ring) {
     const int64_t gi = P.first + i;
     const int sp = advance_neuron<KIND, INTEG, EN>(P, N, i, x, ax) ? 1 : 0;
     if (sp && ring) {
@@ -955,11 +949,6 @@ __device__ __forceinline__ int wide_advance(const PopDev &P, const NetDev &N, in
     record_trace(P, N, ks, gi, x, Model<KIND>::NV);
     if (mon_on<MON>(P)) monitor_state(P, N, ks, i, x, Model<KIND>::NV, sp != 0);
     if (sp) {
-        if (list) {
-            const uint32_t o = atomicAdd(&P.spk_count[ks & 1], 1u);
-            if (o < (uint32_t)P.n) P.spk[o] = (uint32_t)i;
-            else atomicOr(N.flags, FLAG_SPIKELIST_OVERFLOW);
-        }
         if (N.rec_buf) {
             const unsigned long long ro = atomicAdd(N.rec_count, 1ull);
             if (ro < (unsigned long long)N.rec_cap)
@@ -972,7 +961,7 @@ __device__ __forceinline__ int wide_advance(const PopDev &P, const NetDev &N, in
 
 template <int KIND, int INTEG, int MON = 2, int EN = -1>
 __device__ __forceinline__ void wide_window(const PopDev &P, const NetDev &N, int64_t k, int64_t i, WideSmem &S,
-                                            StageSmem &G, float *x, NeuronAux &ax, int nsteps, bool list,
+                                            StageSmem &G, float *x, NeuronAux &ax, int nsteps,
                                             double push_inv_dt) {
     constexpr int ND = Model<KIND>::ND;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
@@ -1010,7 +999,7 @@ __device__ __forceinline__ void wide_window(const PopDev &P, const NetDev &N, in
         while (s1 < nsteps && S.woff[s1 + 1] - S.woff[s0] <= (uint32_t)kStage) ++s1;
         if (s1 == s0) {  // this step alone overflows the stage
             int pf_n = 0;
-            wide_step<KIND, INTEG, MON, EN>(P, N, k + s0, i, S, x, ax, list, push_inv_dt, pf_n, false);
+            wide_step<KIND, INTEG, MON, EN>(P, N, k + s0, i, S, x, ax, false, push_inv_dt, pf_n, false);
             __syncthreads();
             ++s0;
             continue;
@@ -1109,7 +1098,7 @@ __device__ __forceinline__ void wide_window(const PopDev &P, const NetDev &N, in
                         int sp = 0;
                         if (lane == 0) {
                             ordered_sum<ND>(S, S.woff[j] - a0, S.wcnt[j], x, en_mask<EN>(P));
-                            sp = wide_advance<KIND, INTEG, MON, EN>(P, N, k + j, i, S, x, ax, list, ring);
+                            sp = wide_advance<KIND, INTEG, MON, EN>(P, N, k + j, i, S, x, ax, ring);
                         }
                         sp = __shfl_sync(0xffffffffu, sp, 0);
                         if (sp && push_inv_dt > 0.0) push_from(P, N, k + j, gi, lane, 32, push_inv_dt);
@@ -1140,7 +1129,7 @@ __device__ __forceinline__ void wide_window(const PopDev &P, const NetDev &N, in
                 int sp = 0;
                 if (lane == 0) {
                     ordered_sum<ND>(S, o0, c, x, en_mask<EN>(P));
-                    sp = wide_advance<KIND, INTEG, MON, EN>(P, N, ks, i, S, x, ax, list, ring);
+                    sp = wide_advance<KIND, INTEG, MON, EN>(P, N, ks, i, S, x, ax, ring);
                 }
                 sp = __shfl_sync(0xffffffffu, sp, 0);
                 if (sp && push_inv_dt > 0.0) push_from(P, N, ks, gi, lane, 32, push_inv_dt);
@@ -1163,7 +1152,7 @@ __device__ __forceinline__ void wide_window(const PopDev &P, const NetDev &N, in
     }
 }
 
-// Steps k .. k+nsteps-1 of the block's neurons (spike list as in k_update_narrow).
+// Steps k .. k+nsteps-1 of the block's neurons.
 // Populations whose synapses cannot deliver twice in one step take the staged
 // window; the others run step by step.  At most 72 registers a thread: three
 // blocks per SM leave room for one thread-per-neuron block of 256 at 40.
@@ -1174,8 +1163,6 @@ __global__ void __maxnreg__(72) k_update_wide(PopDev P, NetDev N, int rel, int n
     extern __shared__ __align__(32) unsigned char stage_raw[];
     StageSmem &G = *reinterpret_cast<StageSmem *>(stage_raw);
     const int64_t k = cur_step(N, rel);
-    const bool list = nsteps == 1;
-    if (list && blockIdx.x == 0 && threadIdx.x == 0) P.spk_count[(k + 1) & 1] = 0;
     for (int64_t i = blockIdx.x; i < P.n; i += gridDim.x) {
         float x[kMaxVars];
         NeuronAux ax{-1, 0};
@@ -1186,11 +1173,11 @@ __global__ void __maxnreg__(72) k_update_wide(PopDev P, NetDev N, int rel, int n
         }
         __syncthreads();  // S.ring_ok reset before any thread reads it
         if (!P.may_repeat && nsteps <= kMaxWindow) {
-            wide_window<KIND, INTEG, MON, EN>(P, N, k, i, S, G, x, ax, nsteps, list, push_inv_dt);
+            wide_window<KIND, INTEG, MON, EN>(P, N, k, i, S, G, x, ax, nsteps, push_inv_dt);
         } else {
             int pf_n = 0;
             for (int s = 0; s < nsteps; ++s)
-                wide_step<KIND, INTEG, MON, EN>(P, N, k + s, i, S, x, ax, list, push_inv_dt, pf_n, s + 1 < nsteps);
+                wide_step<KIND, INTEG, MON, EN>(P, N, k + s, i, S, x, ax, false, push_inv_dt, pf_n, s + 1 < nsteps);
         }
         if (threadIdx.x == 0) {
             store_state<KIND>(P, i, x);

@@ -146,3 +146,22 @@ def test_gpu_uneven_runs_match_fixture(name):
     if "w_final" in g:
         np.testing.assert_array_equal(sim.weights(), g["w_final"])
     sim.close()
+
+
+@pytest.mark.parametrize("n", [9, 17, 63, 65])
+def test_gpu_short_last_window_matches_fixture(n):
+    """Runs whose length is no multiple of the 8-step window end in a shorter one
+    (one step at 9, 17 and 65), and their flushes of deferred post-synaptic STDP fall
+    between windows: repeated, the result is the reference's."""
+    from edlut_b200.simulation import Simulation
+    net, t, c, nsteps, trace = build_case("cereb_small_rk4")
+    g = load_golden("cereb_small_rk4")
+    sim = Simulation.from_description(net)
+    sim.inject_spikes(t, c)
+    for done in range(0, nsteps, n):
+        sim.run(min(n, nsteps - done))
+    st, ce = sim.spikes()
+    np.testing.assert_array_equal(spike_pairs(st, ce), spike_pairs(g["spike_step"], g["spike_cell"]))
+    if "w_final" in g:
+        np.testing.assert_array_equal(sim.weights(), g["w_final"])
+    sim.close()

@@ -42,7 +42,7 @@ def _stale() -> bool:
 
 
 def _compile_flags():
-    return [*ARCH, "-std=c++17", "-O3", "--fmad=false", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
+    return [*ARCH, "-std=c++17", "-O3", "--fmad=false", "-lineinfo", "-Xfatbin", "-compress-all", "-Xcompiler", "-fPIC,-ffp-contract=off",
             "-diag-suppress", "128", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 
 

@@ -137,12 +137,16 @@ __device__ __forceinline__ void hh_deriv(const PopDev &P, float *x, float *dx, H
     if (x[2] < 0) x[2] = 0.0f;
     if (x[2] > 1) x[2] = 1.0f;
     if (x[3] < 0) x[3] = 0.0f;
-    if ((double)x[3] > 0.72) x[3] = 0.72f;
+    if (x[3] > 0.72f) x[3] = 0.72f;  // the reference compares with the double 0.72, which lies just below 0.72f: the same clamp
     const float V = x[0], m = x[1], h = x[2], n = x[3];
     int pos = (int)((V - kHHMinV) * P.hh_aux);
     if (pos < 0) pos = 0; else if (pos > kHHTable - 1) pos = kHHTable - 1;
-    const float *r = P.hh_table + (size_t)pos * 6;
-    const float am = __ldg(r + 0), bm = __ldg(r + 1), ah = __ldg(r + 2), bh = __ldg(r + 3), an = __ldg(r + 4), bn = __ldg(r + 5);
+    // an entry is one 32-byte sector (kHHRow floats, the last two unused): a 16-byte and
+    // an 8-byte load instead of six gathers
+    const float *r = P.hh_table + (size_t)pos * kHHRow;
+    const float4 ra = __ldg(reinterpret_cast<const float4 *>(r));
+    const float2 rb = __ldg(reinterpret_cast<const float2 *>(r + 4));
+    const float am = ra.x, bm = ra.y, ah = ra.z, bh = ra.w, an = rb.x, bn = rb.y;
     float current = 0.0f;
     if (en & 1) current += x[4] * (eexc - x[0]);
     if (en & 2) current += x[5] * (einh - x[0]);
@@ -165,14 +169,21 @@ __device__ __forceinline__ void hh_deriv(const PopDev &P, float *x, float *dx) {
     hh_deriv<EN>(P, x, dx, R);
 }
 
-// Columns m, h, n of the BDF Jacobian, (f(x) - f(x - eps e_j)) / eps, where x was
-// clamped by the evaluation that gave f(x) = fx and R.  Displacing one gate leaves
-// V, hence the rates, and the other gates' derivatives unchanged: their
-// differences are exactly zero, and dV/dt only needs its displaced term.  The
-// displaced gate is clamped as the full evaluation would clamp it, so every entry
-// is the full evaluation's bit for bit.
-__device__ __forceinline__ void hh_gate_columns(const PopDev &P, const float *x, const float *fx, const HHParts &R,
-                                                float eps, float inv_eps, float *jac) {
+// Non-zero entries of the BDF Jacobian of the HH model, (f(x) - f(x - eps e_j)) / eps,
+// where x was clamped by the evaluation that gave f(x) = fx and R, and neg is
+// f(x - eps e_V).  Displacing one gate leaves V, hence the rates, and the other
+// gates' derivatives unchanged: their differences are exactly zero (the matrix is
+// an arrow: row V, column V and the diagonal), and dV/dt only needs its displaced
+// term.  The displaced gate is clamped as the full evaluation would clamp it, so
+// every entry is the full evaluation's bit for bit.
+struct Arrow4 {
+    float d[4];    // diagonal
+    float row[4];  // row V, columns 1..3
+    float col[4];  // column V, rows 1..3
+};
+
+__device__ __forceinline__ void hh_jacobian(const PopDev &P, const float *x, const float *fx, const HHParts &R,
+                                            const float *neg, float eps, float inv_eps, Arrow4 &A) {
     const float *p = P.p;
     const float gna = p[9], gkd = p[10], ena = p[11], ek = p[12];
     const float V = x[0], m = x[1], h = x[2], n = x[3];
@@ -188,21 +199,19 @@ __device__ __forceinline__ void hh_gate_columns(const PopDev &P, const float *x,
     const float dh2 = R.ah * (1.0f - h2) - R.bh * h2;
     float n2 = n - eps;
     if (n2 < 0) n2 = 0.0f;
-    if ((double)n2 > 0.72) n2 = 0.72f;
+    if (n2 > 0.72f) n2 = 0.72f;
     const float dn0 = (R.sA + gkd * n2 * n2 * n2 * n2 * (ek - V)) * P.inv_c_m;
     const float dn3 = R.an * (1.0f - n2) - R.bn * n2;
-    jac[0 * 4 + 1] = (fx[0] - dm0) * inv_eps;
-    jac[1 * 4 + 1] = (fx[1] - dm1) * inv_eps;
-    jac[2 * 4 + 1] = 0.0f;
-    jac[3 * 4 + 1] = 0.0f;
-    jac[0 * 4 + 2] = (fx[0] - dh0) * inv_eps;
-    jac[1 * 4 + 2] = 0.0f;
-    jac[2 * 4 + 2] = (fx[2] - dh2) * inv_eps;
-    jac[3 * 4 + 2] = 0.0f;
-    jac[0 * 4 + 3] = (fx[0] - dn0) * inv_eps;
-    jac[1 * 4 + 3] = 0.0f;
-    jac[2 * 4 + 3] = 0.0f;
-    jac[3 * 4 + 3] = (fx[3] - dn3) * inv_eps;
+    A.d[0] = (fx[0] - neg[0]) * inv_eps;
+    A.row[1] = (fx[0] - dm0) * inv_eps;
+    A.row[2] = (fx[0] - dh0) * inv_eps;
+    A.row[3] = (fx[0] - dn0) * inv_eps;
+    A.col[1] = (fx[1] - neg[1]) * inv_eps;
+    A.col[2] = (fx[2] - neg[2]) * inv_eps;
+    A.col[3] = (fx[3] - neg[3]) * inv_eps;
+    A.d[1] = (fx[1] - dm1) * inv_eps;
+    A.d[2] = (fx[2] - dh2) * inv_eps;
+    A.d[3] = (fx[3] - dn3) * inv_eps;
 }
 
 template <int KIND> struct Model;
@@ -287,6 +296,73 @@ __device__ __forceinline__ bool invermat(const float *a, float *ainv) {
     return true;
 }
 
+// a = A^-1 r for an arrow matrix A by the operations of invermat<4> (Gauss-Jordan
+// inverse, then the product), leaving out those on structural zeros: x + 0 k is x
+// and 0 + y is y while k is finite, so the values are the general path's as long as
+// no pivot's reciprocal and no coefficient is infinite or NaN -- and one that is
+// stays in its entry of the inverse and shows in a.  Returns false then (also for
+// a zero pivot, whose row swap needs the general path).
+__device__ __forceinline__ bool arrow_solve(const Arrow4 &A, const float *r, float *a) {
+    float l[4][4];
+    float b1 = A.row[1], b2 = A.row[2], b3 = A.row[3];
+    float inv = 1.0f / A.d[0];
+    b1 *= inv; b2 *= inv; b3 *= inv;
+    l[0][0] = inv;
+    const float c1 = -A.col[1], c2 = -A.col[2], c3 = -A.col[3];
+    float m11 = A.d[1] + b1 * c1, m12 = b2 * c1, m13 = b3 * c1;
+    float m21 = b1 * c2, m22 = A.d[2] + b2 * c2, m23 = b3 * c2;
+    float m31 = b1 * c3, m32 = b2 * c3, m33 = A.d[3] + b3 * c3;
+    l[1][0] = inv * c1;
+    l[2][0] = inv * c2;
+    l[3][0] = inv * c3;
+    inv = 1.0f / m11;
+    m12 *= inv; m13 *= inv; l[1][0] *= inv; l[1][1] = inv;
+    float k = -b1;
+    b2 += m12 * k; b3 += m13 * k; l[0][0] += l[1][0] * k; l[0][1] = inv * k;
+    k = -m21;
+    m22 += m12 * k; m23 += m13 * k; l[2][0] += l[1][0] * k; l[2][1] = inv * k;
+    k = -m31;
+    m32 += m12 * k; m33 += m13 * k; l[3][0] += l[1][0] * k; l[3][1] = inv * k;
+    inv = 1.0f / m22;
+    m23 *= inv; l[2][0] *= inv; l[2][1] *= inv; l[2][2] = inv;
+    k = -b2;
+    b3 += m23 * k; l[0][0] += l[2][0] * k; l[0][1] += l[2][1] * k; l[0][2] = inv * k;
+    k = -m12;
+    m13 += m23 * k; l[1][0] += l[2][0] * k; l[1][1] += l[2][1] * k; l[1][2] = inv * k;
+    k = -m32;
+    m33 += m23 * k; l[3][0] += l[2][0] * k; l[3][1] += l[2][1] * k; l[3][2] = inv * k;
+    inv = 1.0f / m33;
+    l[3][0] *= inv; l[3][1] *= inv; l[3][2] *= inv; l[3][3] = inv;
+    k = -b3;
+    l[0][0] += l[3][0] * k; l[0][1] += l[3][1] * k; l[0][2] += l[3][2] * k; l[0][3] = inv * k;
+    k = -m13;
+    l[1][0] += l[3][0] * k; l[1][1] += l[3][1] * k; l[1][2] += l[3][2] * k; l[1][3] = inv * k;
+    k = -m23;
+    l[2][0] += l[3][0] * k; l[2][1] += l[3][1] * k; l[2][2] += l[3][2] * k; l[2][3] = inv * k;
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+        float v = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) v += l[z][t] * r[t];
+        a[z] = v;
+    }
+    return fabsf(a[0]) + fabsf(a[1]) + fabsf(a[2]) + fabsf(a[3]) < __int_as_float(0x7f800000);
+}
+
+// The general path for an arrow matrix (rare: see arrow_solve).
+static __device__ __noinline__ bool arrow_solve_general(const Arrow4 &A, const float *r, float *a) {
+    float J[16] = {A.d[0], A.row[1], A.row[2], A.row[3], A.col[1], A.d[1], 0.0f, 0.0f,
+                   A.col[2], 0.0f, A.d[2], 0.0f, A.col[3], 0.0f, 0.0f, A.d[3]};
+    float iJ[16];
+    if (!invermat<4>(J, iJ)) return false;
+    for (int z = 0; z < 4; ++z) {
+        float v = 0.0f;
+        for (int t = 0; t < 4; ++t) v += iJ[z * 4 + t] * r[t];
+        a[z] = v;
+    }
+    return true;
+}
+
 // Per-neuron BDF history, SoA in global memory: D[q][v][n], P[q][v][n].
 struct BdfRef {
     float *D, *Pv;
@@ -358,47 +434,96 @@ __device__ __forceinline__ bool integrate(const PopDev &P, float *x, int refr, i
         decay<ND, EN>(P, pr);
         const float *co = P.bdf_coef[st];
         float hist[6][ND];
-        for (int q = 1; q < st; ++q)
+        for (int q = KIND == KIND_HH ? 2 : 1; q < st; ++q)
 #pragma unroll
             for (int j = 0; j < ND; ++j) hist[q - 1][j] = H.pv(q - 1, j, ND);
         float epsi = 1.0f;
         int k = 0;
         const float eps_j = dt * 0.1f;
         const float inv_eps = 1.0f / eps_j;
-        HHParts R;
+        if constexpr (KIND == KIND_HH) {
+            const float cd = co[0] * dt;
+            // Bound by the serial chain of one warp (small populations) or by issue (100,000
+            // neurons).  The history term of order 2 stays in registers: hist is indexed at
+            // run time and lives in local memory, whose loads in every iteration cost the
+            // most (us a step at 3,001 / 100,000 neurons: 20.8 / 48.7 -> 14.5 / 33.4); the
+            // arrow elimination and the 32-byte table rows gave 27.1 / 57.3 -> 20.8 / 48.7.
+            float h0[ND];
+#pragma unroll
+            for (int j = 0; j < ND; ++j) h0[j] = st > 1 ? co[2] * H.pv(0, j, ND) : 0.0f;
+            bool general = false;
+            HHParts R;
+            while (epsi > 1e-6 && k < 10) {
+                hh_deriv<EN>(P, pr, aux, R);
+#pragma unroll
+                for (int j = 0; j < ND; ++j) {
+                    c[j] = cd * aux[j] + co[1] * x[j];
+                    if (st > 1) c[j] += h0[j];
+                }
+                for (int q = 2; q < st; ++q)  // orders above 2
+#pragma unroll
+                    for (int j = 0; j < ND; ++j) c[j] += co[q + 1] * hist[q - 1][j];
+#pragma unroll
+                for (int j = 0; j < ND; ++j) c[j] = pr[j] - c[j];
+                // Jacobian: one-sided difference at eps = 0.1 dt (BDFn.h:704-724).  Its
+                // base point is f(pr), already in aux: deriv clamps its argument in
+                // place before evaluating and clamping twice changes nothing, so
+                // evaluating it again would give the same values bit for bit.
+                float tmp[NV], neg[NV];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) tmp[v] = pr[v];
+                tmp[0] -= eps_j;
+                hh_deriv<EN>(P, tmp, neg);
+                Arrow4 A;
+                hh_jacobian(P, pr, aux, R, neg, eps_j, inv_eps, A);
+                A.d[0] = cd * A.d[0] - 1;
+#pragma unroll
+                for (int j = 1; j < ND; ++j) {
+                    A.d[j] = cd * A.d[j] - 1;
+                    A.row[j] = cd * A.row[j];
+                    A.col[j] = cd * A.col[j];
+                }
+                bool ok;
+                if (!general) {
+                    ok = arrow_solve(A, c, p1);
+                } else {
+                    ok = arrow_solve_general(A, c, p1);
+                    if (!ok) return false;
+                }
+                general = !ok;  // this iteration again, on the general path
+                if (ok) {
+                    float mx = 0.0f;
+#pragma unroll
+                    for (int z = 0; z < ND; ++z) {
+                        p1[z] += pr[z];
+                        const float d = fabsf(p1[z] - pr[z]);
+                        if (d > mx) mx = d;
+                        pr[z] = p1[z];
+                    }
+                    epsi = mx;
+                    k++;
+                }
+            }
+        } else
         while (epsi > 1e-6 && k < 10) {
-            if constexpr (KIND == KIND_HH) hh_deriv<EN>(P, pr, aux, R);
-            else M::template deriv<EN>(P, pr, aux, rf);
+            M::template deriv<EN>(P, pr, aux, rf);
 #pragma unroll
             for (int j = 0; j < ND; ++j) {
                 c[j] = co[0] * dt * aux[j] + co[1] * x[j];
                 for (int q = 1; q < st; ++q) c[j] += co[q + 1] * hist[q - 1][j];
             }
-            // Jacobian: one-sided difference at eps = 0.1 dt (BDFn.h:704-724).  Its
-            // base point is f(pr), already in aux: deriv clamps its argument in
-            // place before evaluating (HH) and clamping twice changes nothing, so
-            // evaluating it again would give the same values bit for bit.
-            if constexpr (KIND == KIND_HH) {
-                float tmp[NV], neg[NV];
+            // Jacobian: one-sided difference at eps = 0.1 dt (BDFn.h:704-724), based on
+            // f(pr), already in aux
+            float tmp[NV], neg[NV];
+            const float *pos = aux;
+#pragma unroll
+            for (int j = 0; j < ND; ++j) {
 #pragma unroll
                 for (int v = 0; v < NV; ++v) tmp[v] = pr[v];
-                tmp[0] -= eps_j;
+                tmp[j] -= eps_j;
                 M::template deriv<EN>(P, tmp, neg, rf);
 #pragma unroll
-                for (int z = 0; z < ND; ++z) jac[z * ND] = (aux[z] - neg[z]) * inv_eps;
-                hh_gate_columns(P, pr, aux, R, eps_j, inv_eps, jac);
-            } else {
-                float tmp[NV], neg[NV];
-                const float *pos = aux;
-#pragma unroll
-                for (int j = 0; j < ND; ++j) {
-#pragma unroll
-                    for (int v = 0; v < NV; ++v) tmp[v] = pr[v];
-                    tmp[j] -= eps_j;
-                    M::template deriv<EN>(P, tmp, neg, rf);
-#pragma unroll
-                    for (int z = 0; z < ND; ++z) jac[z * ND + j] = (pos[z] - neg[z]) * inv_eps;
-                }
+                for (int z = 0; z < ND; ++z) jac[z * ND + j] = (pos[z] - neg[z]) * inv_eps;
             }
 #pragma unroll
             for (int z = 0; z < ND; ++z)
@@ -429,18 +554,20 @@ __device__ __forceinline__ bool integrate(const PopDev &P, float *x, int refr, i
         if (st < P.bdf_order) st++;
         bdf_state = st;
 #pragma unroll
-        for (int j = 0; j < ND; ++j) {
-            float dq[7];
-            for (int q = 0; q < st; ++q) dq[q] = H.d(q, j, ND);
-            for (int q = st - 1; q > 0; --q) dq[q] = -dq[q - 1];
-            dq[0] = pr[j] - x[j];
-            for (int q = 1; q < st; ++q) dq[q] += dq[q - 1];
-            for (int q = 0; q < st; ++q) H.d(q, j, ND) = dq[q];
+        for (int j = 0; j < ND; ++j) {  // D[q] <- D'[q - 1] - D[q - 1], D'[0] the new difference
+            float now = pr[j] - x[j], old = H.d(0, j, ND);
+            H.d(0, j, ND) = now;
+            for (int q = 1; q < st; ++q) {
+                const float next = H.d(q, j, ND);
+                now = -old + now;
+                old = next;
+                H.d(q, j, ND) = now;
+            }
         }
         if (st > 1) {
             for (int q = st - 2; q > 0; --q)
 #pragma unroll
-                for (int j = 0; j < ND; ++j) H.pv(q, j, ND) = hist[q - 1][j];
+                for (int j = 0; j < ND; ++j) H.pv(q, j, ND) = H.pv(q - 1, j, ND);
 #pragma unroll
             for (int j = 0; j < ND; ++j) H.pv(0, j, ND) = x[j];
         }

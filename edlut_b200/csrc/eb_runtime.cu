@@ -406,7 +406,9 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
                 init[1] = v[0] / (v[0] + v[1]);
                 init[2] = v[2] / (v[2] + v[3]);
                 init[3] = v[4] / (v[4] + v[5]);
-                if ((rc = upload(this, (float **)&D.hh_table, hh))) return rc;
+                std::vector<float> rows((size_t)kHHTable * kHHRow, 0.0f);
+                for (int64_t e = 0; e < kHHTable; ++e) std::copy_n(hh.data() + e * 6, 6, rows.data() + e * kHHRow);
+                if ((rc = upload(this, (float **)&D.hh_table, rows))) return rc;
                 nmda = make_nmda_table(pr[0], pr[1], &D.nmda_aux);
             }
             if ((rc = upload(this, (float **)&D.nmda_table, nmda))) return rc;

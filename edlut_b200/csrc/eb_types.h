@@ -17,6 +17,7 @@ constexpr int kPostGraph = 64;
 constexpr int kNmdaTable = 256;
 constexpr int kExptTable = 1024 * 16;
 constexpr int kHHTable = 1024 * 256;
+constexpr int kHHRow = 8;  // floats from one entry of the device's HH rate table to the next (6 used)
 
 // Device error flags (ORed into NetDev::flags).
 constexpr uint32_t FLAG_BUCKET_OVERFLOW = 1u;

@@ -481,7 +481,7 @@ __device__ __forceinline__ void update_narrow_tile(const PopDev &P, const NetDev
     }
 }
 
-// Steps k .. k+nsteps-1 of one tile, the state in registers between them.
+// Steps k .. k+nsteps-1 of npw neurons a warp, the state in registers between them.
 // push_inv_dt > 0: also fan out the spikes (1 / step, for arrival_step).
 // HH under BDF holds the Newton state (Jacobian, inverse, history) in about 120
 // registers, which leaves 2 blocks per SM; bounded to 3 blocks (80 registers, a
@@ -496,10 +496,11 @@ constexpr int narrow_min_blocks(int kind, int integ) {
 
 template <int KIND, int INTEG, int EN, int MON>
 __global__ void __launch_bounds__(kNarrowTile, narrow_min_blocks(KIND, INTEG)) k_update_narrow(PopDev P, NetDev N, int rel, int nsteps,
-                                                                double push_inv_dt) {
+                                                                double push_inv_dt, int npw) {
     const int64_t k = cur_step(N, rel);
-    const int64_t i = (int64_t)blockIdx.x * kNarrowTile + threadIdx.x;
-    const bool active = i < P.n;
+    const int lane = threadIdx.x & 31;
+    const int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * npw + lane;
+    const bool active = lane < npw && i < P.n;
     float x[kMaxVars];
     NeuronAux ax{-1, 0};
     if (active) {

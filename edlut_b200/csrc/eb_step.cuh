@@ -99,12 +99,14 @@ __device__ __forceinline__ void stdp_post(const NetDev &N, SynRec &r, double t) 
 // factors of the interval ending at each spike; in global memory (RingGlobal) or
 // staged in shared memory (RingSmem).
 struct RingGlobal {
+    static constexpr bool kLooksAhead = true;
     const double *t;     // the neuron's kPostRing times
     const DecayPair *f;  // and factors
     __device__ double time(uint32_t slot) const { return t[slot]; }
     __device__ DecayPair fac(uint32_t slot) const { return f[slot]; }
 };
 struct RingSmem {
+    static constexpr bool kLooksAhead = false;
     const double *t;
     const DecayPair *f;
     __device__ double time(uint32_t slot) const { return t[slot]; }
@@ -112,14 +114,26 @@ struct RingSmem {
 };
 
 // Apply to r the ring's spikes after r.last, oldest first, as stdp_post would one
-// by one.  Spike times increase with the spike number, so the first pending one
-// is found by bisection.  After the first, r.last is the previous spike, so each
+// by one.  Spike times increase with the spike number, so the first pending one is
+// found by bisection -- after a look at the newest kRingNewest at once when the ring
+// is in global memory, where each probe waits for the one before and few spikes are
+// pending as a rule.  After the first, r.last is the previous spike, so each
 // update's elapsed time -- and its two table lookups -- are the interval's: they
 // come from the factor ring when r follows the ring's rule (rule >= 0).
+constexpr uint32_t kRingNewest = 4;
+
 template <class Ring>
 __device__ __forceinline__ void apply_pending(const NetDev &N, const Ring &ring, uint32_t c, int rule, SynRec &r) {
     const uint32_t lim = c < (uint32_t)kPostRing ? c : (uint32_t)kPostRing;
     uint32_t lo = c - lim, hi = c;  // first spike number in [lo, hi) with time > r.last
+    if constexpr (Ring::kLooksAhead) {
+        uint32_t n = 0;  // pending among the newest
+#pragma unroll
+        for (uint32_t q = 1; q <= kRingNewest; ++q)
+            if (q <= lim && ring.time((c - q) % kPostRing) > r.last) n = q;
+        hi = c - n;
+        if (n < kRingNewest) lo = hi;
+    }
     while (lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
         if (ring.time(mid % kPostRing) > r.last) hi = mid;
@@ -368,17 +382,46 @@ __device__ __forceinline__ void bucket_put(const NetDev &N, int64_t ka, double a
     }
 }
 
-// One spike of population P at step k (update time t_k): the block's threads
-// cover the source's out-synapses (sorted by delay, then target).
-// Fan-out of source neuron src's spike at step k: lanes lane, lane + width, ...
-// of the caller's group take its out-synapses.
+// Fan-out of source neuron src's spike at step k: lanes lane, lane + width, ... of
+// the caller's group take its out-synapses (sorted by delay, then target), each
+// BATCH at a time: a delivery is a chain of three dependent accesses (synapse, bucket,
+// reservation), and a source's deliveries are independent.
+template <int BATCH = 1>
 __device__ __forceinline__ void push_from(const PopDev &P, const NetDev &N, int64_t k, int64_t src, int lane, int width,
                                           double inv_dt) {
     const double tk = P.kind == KIND_POISSON ? N.tgen[k] : N.tstep[k];  // generators spike on their own grid
     const int64_t o0 = N.out_ptr[src], o1 = N.out_ptr[src + 1];
-    for (int64_t o = o0 + lane; o < o1; o += width) {
-        const double a = tk + (double)N.out_units[o] * 0.0001;
-        bucket_put(N, arrival_step(N, a, k + 1, inv_dt), a, o);
+    for (int64_t o = o0 + lane; o < o1; o += BATCH * width) {
+        uint32_t tg[BATCH];
+        Arrival v[BATCH];
+        int slot[BATCH];
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            const int64_t q = o + u * width;
+            if (q >= o1) continue;
+            tg[u] = N.out_tgt[q];
+            v[u].a = tk + (double)N.out_units[q] * 0.0001;
+            v[u].spos = (uint32_t)q;
+            v[u].tpos = N.out_tpos[q];
+        }
+        uint32_t capg[BATCH];
+        int64_t base[BATCH];
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            if (o + u * width >= o1) continue;
+            capg[u] = N.cap[tg[u]];
+            base[u] = N.cap_base[tg[u]];
+            slot[u] = (int)(arrival_step(N, v[u].a, k + 1, inv_dt) & (N.R - 1));
+        }
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u)
+            if (o + u * width < o1) tg[u] = atomicAdd(N.cnt + (int64_t)slot[u] * N.n_neurons + tg[u], 1u);
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            if (o + u * width >= o1) continue;
+            if (tg[u] < capg[u]) N.rec[(int64_t)slot[u] * N.cap_total + base[u] + tg[u]] = v[u];
+            else atomicOr(N.flags, FLAG_BUCKET_OVERFLOW);
+        }
     }
 }
 
@@ -390,6 +433,7 @@ __device__ __forceinline__ void push_spike(const PopDev &P, const NetDev &N, int
 // buckets of steps >= k+1, which no kernel of this step reads, so the spiking
 // warp delivers it at once instead of a separate launch after the update.  The
 // warp takes its spiking lanes one at a time, lanes over the out-synapses.
+template <int BATCH = 1>
 __device__ __forceinline__ void warp_push(const PopDev &P, const NetDev &N, int64_t k, int64_t i, bool sp,
                                           double inv_dt) {
     unsigned m = __ballot_sync(0xffffffffu, sp);
@@ -398,67 +442,93 @@ __device__ __forceinline__ void warp_push(const PopDev &P, const NetDev &N, int6
         const int l = __ffs(m) - 1;
         m &= m - 1u;
         const int64_t src = P.first + __shfl_sync(0xffffffffu, i, l);
-        push_from(P, N, k, src, lane, 32, inv_dt);
+        push_from<BATCH>(P, N, k, src, lane, 32, inv_dt);
     }
 }
+
+// Asynchronous global -> shared copies (cp.async), complete at cp_async_wait_all
+// (and a barrier of the threads that read them).
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // ----------------------------------------------------------- narrow update --
 // One thread per neuron.  Arrivals of this step are sorted in registers
 // (insertion sort; at most 16 in the fast path) and folded in order.
 constexpr int kLocalSort = 16;
-constexpr int kNarrowTile = 256;
+constexpr int kNarrowTile = 256;   // threads of the persistent kernel's tiles
+constexpr int kNarrowBlock = 64;   // most threads of a block of k_update_narrow
+// Steps of one launch (the runtime's window length).
+constexpr int kMaxWindow = 8;
 
-// One step of neuron i (lanes with active unset only join the warp collectives);
-// x and ax hold its state, loaded and stored by the caller.
-template <int KIND, int INTEG, int EN = -1, int MON = 2>
-__device__ __forceinline__ void narrow_step(const PopDev &P, const NetDev &N, int64_t k, int64_t i, bool active,
-                                            float *x, NeuronAux &ax, bool list, double push_inv_dt) {
-    constexpr int ND = Model<KIND>::ND;
-    bool sp = false;
-    uint32_t c = 0;
-    if (active) {
-        const int64_t gi = P.first + i;
-        const int slot = (int)(k & (N.R - 1));
-        uint32_t *cp = N.cnt + (int64_t)slot * N.n_neurons + gi;
-        c = *cp;
-        if (c) {
-            *cp = 0;
-            const uint32_t capg = N.cap[gi];
-            if (c > capg) { atomicOr(N.flags, FLAG_BUCKET_OVERFLOW); c = capg; }
-            Arrival *r = N.rec + (int64_t)slot * N.cap_total + N.cap_base[gi];
-            if (c == 1) {
-                apply_arrival<ND, MON>(P, N, k, i, r[0], x);
-            } else if (c <= kLocalSort) {
-                Arrival loc[kLocalSort];
-                for (uint32_t a = 0; a < c; ++a) {
-                    Arrival v = r[a];
-                    int b = (int)a - 1;
-                    while (b >= 0 && arr_less(v, loc[b])) { loc[b + 1] = loc[b]; --b; }
-                    loc[b + 1] = v;
-                }
-                for (uint32_t a = 0; a < c; ++a) apply_arrival<ND, MON>(P, N, k, i, loc[a], x);
-            } else {
-                for (uint32_t a = 1; a < c; ++a) {  // in-place insertion sort (rare path)
-                    Arrival v = r[a];
-                    int b = (int)a - 1;
-                    while (b >= 0 && arr_less(v, r[b])) { r[b + 1] = r[b]; --b; }
-                    r[b + 1] = v;
-                }
-                for (uint32_t a = 0; a < c; ++a) apply_arrival<ND, MON>(P, N, k, i, r[a], x);
+// The arrivals of step k at neuron i, from its bucket, onto x; returns their number.
+template <int ND, int MON>
+__device__ __forceinline__ uint32_t narrow_fold(const PopDev &P, const NetDev &N, int64_t k, int64_t i, float *x) {
+    const int64_t gi = P.first + i;
+    const int slot = (int)(k & (N.R - 1));
+    uint32_t *cp = N.cnt + (int64_t)slot * N.n_neurons + gi;
+    uint32_t c = *cp;
+    if (c) {
+        *cp = 0;
+        const uint32_t capg = N.cap[gi];
+        if (c > capg) { atomicOr(N.flags, FLAG_BUCKET_OVERFLOW); c = capg; }
+        Arrival *r = N.rec + (int64_t)slot * N.cap_total + N.cap_base[gi];
+        if (c == 1) {
+            apply_arrival<ND, MON>(P, N, k, i, r[0], x);
+        } else if (c <= kLocalSort) {
+            Arrival loc[kLocalSort];
+            for (uint32_t a = 0; a < c; ++a) {
+                Arrival v = r[a];
+                int b = (int)a - 1;
+                while (b >= 0 && arr_less(v, loc[b])) { loc[b + 1] = loc[b]; --b; }
+                loc[b + 1] = v;
             }
+            for (uint32_t a = 0; a < c; ++a) apply_arrival<ND, MON>(P, N, k, i, loc[a], x);
+        } else {
+            for (uint32_t a = 1; a < c; ++a) {  // in-place insertion sort (rare path)
+                Arrival v = r[a];
+                int b = (int)a - 1;
+                while (b >= 0 && arr_less(v, r[b])) { r[b + 1] = r[b]; --b; }
+                r[b + 1] = v;
+            }
+            for (uint32_t a = 0; a < c; ++a) apply_arrival<ND, MON>(P, N, k, i, r[a], x);
         }
-        sp = advance_neuron<KIND, INTEG, EN>(P, N, i, x, ax);
-        record_trace(P, N, k, gi, x, Model<KIND>::NV);
-        if (mon_on<MON>(P)) monitor_state(P, N, k, i, x, Model<KIND>::NV, sp);
-        if (sp && P.post_t) note_post_spike(P, N, i, k);
     }
-    // delivered-event counter: one atomic per warp
+    return c;
+}
+
+// Delivered-event counter: one atomic per warp.
+__device__ __forceinline__ void count_events(const PopDev &P, uint32_t c) {
     if (__any_sync(0xffffffffu, c != 0)) {
         unsigned long long cw = c;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cw += __shfl_down_sync(0xffffffffu, cw, o);
         if ((threadIdx.x & 31) == 0 && cw) atomicAdd(P.events, cw);
     }
+}
+
+// One step of neuron i (lanes with active unset only join the warp collectives);
+// x and ax hold its state, loaded and stored by the caller.
+template <int KIND, int INTEG, int EN = -1, int MON = 2>
+__device__ __forceinline__ void narrow_step(const PopDev &P, const NetDev &N, int64_t k, int64_t i, bool active,
+                                            float *x, NeuronAux &ax, bool list, double push_inv_dt) {
+    bool sp = false;
+    uint32_t c = 0;
+    if (active) {
+        c = narrow_fold<Model<KIND>::ND, MON>(P, N, k, i, x);
+        sp = advance_neuron<KIND, INTEG, EN>(P, N, i, x, ax);
+        record_trace(P, N, k, P.first + i, x, Model<KIND>::NV);
+        if (mon_on<MON>(P)) monitor_state(P, N, k, i, x, Model<KIND>::NV, sp);
+        if (sp && P.post_t) note_post_spike(P, N, i, k);
+    }
+    count_events(P, c);
     compact_spikes(P, N, k, i, sp, list);
     if (push_inv_dt > 0.0) warp_push(P, N, k, i, sp, push_inv_dt);
 }
@@ -481,8 +551,196 @@ __device__ __forceinline__ void update_narrow_tile(const PopDev &P, const NetDev
     }
 }
 
-// Steps k .. k+nsteps-1 of npw neurons a warp, the state in registers between them.
+// ------------------------------------------------------ staged narrow window --
+// The steps of one launch for the neurons of one warp, with the window's arrivals
+// taken in at once.  Every bucket of the window is final when the launch starts, so
+// the warp reads the counts of all its steps, copies the arrivals of as many
+// consecutive steps as its stage holds into shared memory, each lane its neuron's,
+// step by step, and sorts each step's few in delivery order.  That leaves three
+// dependent global accesses (count, arrival, synapse) a window where the per-step
+// fold waited for them at every step, one arrival after the other.
+//   Populations without plastic inputs: all staged arrivals' weights are fetched
+// together, a step's fold only reads shared memory.
+//   With plastic inputs: a step's arrivals are dealt out to the lanes, whoever's
+// neuron they reach, and every lane catches its synapse up on the target's
+// post-synaptic spikes, takes the weight and applies the pre-synaptic update;
+// the owner then adds the weights in order.  Synapses are independent unless one
+// delivers twice in the step (input neurons only): then the step folds serially.
+// A step with more arrivals than the stage holds runs on the per-step path.
+//   Bound by the latency of the warp's chain: 1,000 LIF neurons, 3,000 steps 4.37 ->
+// 3.32 ms; 2,501 AdEx neurons with STDP, 500 steps 3.62 -> 2.42 ms; HH, 3,001 neurons
+// 12.9 -> 11.8 us a step, 100,000 29.7 -> 28.2.  Large LIF and AdEx populations are
+// bound by issue at 40 registers, where the staging spills 250 bytes: they keep the
+// per-step fold (250,000 granule cells 5.98 us a step, 6.16 staged).
+template <int CAP>
+struct NarrowStage {
+    Arrival arr[CAP];
+    float w[CAP];
+    uint16_t list[CAP];  // a step's arrivals: owner lane << 8 | position
+    uint8_t ty[CAP];
+};
+// Arrivals of a warp's stage: HH under BDF runs few, long-lived warps of neurons with
+// many inputs; the others keep the shared memory of 48 warps an SM below half of it.
+__host__ __device__ constexpr int narrow_stage(int kind) { return kind == KIND_HH ? 128 : 64; }
+static_assert(kMaxWindow <= 8, "a lane packs a window's counts into 8 bytes");
+
+template <int KIND, int INTEG, int EN, int MON, bool SMALL, int CAP>
+__device__ __forceinline__ void narrow_window(const PopDev &P, const NetDev &N, int64_t k, int64_t i, bool active,
+                                              float *x, NeuronAux &ax, int nsteps, double push_inv_dt,
+                                              NarrowStage<CAP> &S) {
+    constexpr int ND = Model<KIND>::ND;
+    constexpr unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t gi = P.first + i;
+    const bool plastic = P.post_t != nullptr;
+    // counts of the steps not yet run, a byte each (255: that many or more), next step lowest
+    unsigned long long pk = 0;
+    uint32_t capg = 0;
+    const Arrival *rec = nullptr;
+    if (active) {
+#pragma unroll
+        for (int s = 0; s < kMaxWindow; ++s)
+            if (s < nsteps) {
+                const uint32_t c = N.cnt[(int64_t)((k + s) & (N.R - 1)) * N.n_neurons + gi];
+                pk |= (unsigned long long)(c < 255u ? c : 255u) << (8 * s);
+            }
+        if (pk) {
+            capg = N.cap[gi];
+            rec = N.rec + N.cap_base[gi];
+        }
+    }
+    int staged = 0;      // steps left of the staged chunk
+    uint32_t pos = 0;    // this lane's next staged arrival
+    for (int s = 0; s < nsteps; ++s) {
+        const int64_t ks = k + s;
+        if (staged == 0) {
+
+            if (__any_sync(full, pk != 0)) {
+                int len = nsteps - s;
+                uint32_t tot, incl, T;
+                for (;;) {
+                    tot = 0;
+                    for (int q = 0; q < len; ++q) {
+                        const uint32_t c = (uint32_t)(pk >> (8 * q)) & 255u;
+                        tot += c == 255u || c > capg ? CAP + 1 : c;
+                    }
+                    incl = tot;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t u = __shfl_up_sync(full, incl, o);
+                        if (lane >= o) incl += u;
+                    }
+                    T = __shfl_sync(full, incl, 31);
+                    if (T <= (uint32_t)CAP || len == 1) break;
+                    len >>= 1;
+                }
+                staged = len;
+                pos = incl - tot;
+                const bool direct = T > (uint32_t)CAP;  // this step alone overflows the stage (or a bucket)
+                if (direct) {
+                    count_events(P, active ? narrow_fold<ND, MON>(P, N, ks, i, x) : 0u);
+                    pk &= ~255ull;
+                } else if (T) {
+                    __syncwarp();  // every lane is done with the last chunk
+                    uint32_t j = pos;
+                    if (tot)
+                        for (int q = 0; q < len; ++q) {
+                            const uint32_t c = (uint32_t)(pk >> (8 * q)) & 255u;
+                            if (!c) continue;
+                            const int slot = (int)((ks + q) & (N.R - 1));
+                            const Arrival *r = rec + (int64_t)slot * N.cap_total;
+                            for (uint32_t a = 0; a < c; ++a) cp_async16(&S.arr[j++], r + a);
+                            N.cnt[(int64_t)slot * N.n_neurons + gi] = 0;
+                        }
+                    cp_async_commit();
+                    if (lane == 0) atomicAdd(P.events, (unsigned long long)T);
+                    cp_async_wait_all();
+                    j = pos;
+                    if (tot)
+                        for (int q = 0; q < len; ++q) {  // each step's arrivals in delivery order
+                            const uint32_t c = (uint32_t)(pk >> (8 * q)) & 255u;
+                            for (uint32_t a = 1; a < c; ++a) {
+                                const Arrival v = S.arr[j + a];
+                                uint32_t b = a;
+                                while (b > 0 && arr_less(v, S.arr[j + b - 1])) { S.arr[j + b] = S.arr[j + b - 1]; --b; }
+                                if (b != a) S.arr[j + b] = v;
+                            }
+                            j += c;
+                        }
+                    __syncwarp();
+                    for (uint32_t e = lane; e < T; e += 32) {
+                        const SynRec *r = N.syn + S.arr[e].tpos;
+                        if (plastic) {
+                            prefetch_l1(r);
+                        } else {
+                            S.w[e] = r->w;
+                            S.ty[e] = r->stype;
+                        }
+                    }
+                    __syncwarp();
+                }
+            } else {
+                staged = nsteps - s;  // no arrival in the rest of the window
+            }
+        }
+        --staged;
+        const uint32_t c = (uint32_t)pk & 255u;
+        pk >>= 8;
+        bool serial = false;  // a synapse delivers twice in this step
+        if (plastic && __any_sync(full, c != 0)) {
+            if (P.may_repeat) {
+                bool twice = false;
+                for (uint32_t a = 1; a < c; ++a)
+                    for (uint32_t b = 0; b < a; ++b) twice = twice || S.arr[pos + a].spos == S.arr[pos + b].spos;
+                serial = __any_sync(full, twice);
+            }
+            if (!serial) {
+                uint32_t incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t u = __shfl_up_sync(full, incl, o);
+                    if (lane >= o) incl += u;
+                }
+                const uint32_t T = __shfl_sync(full, incl, 31);
+                for (uint32_t a = 0; a < c; ++a) S.list[incl - c + a] = (uint16_t)(lane << 8 | (pos + a));
+                __syncwarp();
+                for (uint32_t e = lane; e < T; e += 32) {
+                    const uint32_t at = S.list[e];
+                    const Arrival v = S.arr[at & 255u];
+                    SynRec r = N.syn[v.tpos];
+                    if (r.rule >= 0) apply_pending_post(P, N, i - lane + (at >> 8), r);
+                    S.w[at & 255u] = r.w;
+                    S.ty[at & 255u] = r.stype;
+                    if (r.rule >= 0) stdp_pre(N, v.tpos, r, v.a);
+                }
+                __syncwarp();
+            }
+        }
+        bool sp = false;
+        if (active) {
+            if (serial) {
+                for (uint32_t a = 0; a < c; ++a) apply_arrival<ND, MON>(P, N, ks, i, S.arr[pos + a], x);
+            } else {
+                for (uint32_t a = 0; a < c; ++a) {
+                    add_conductance<ND>(x, S.ty[pos + a], S.w[pos + a]);
+                    if (mon_on<MON>(P)) monitor_delivery(P, N, ks, i, S.arr[pos + a], S.ty[pos + a], S.w[pos + a]);
+                }
+            }
+            pos += c;
+            sp = advance_neuron<KIND, INTEG, EN>(P, N, i, x, ax);
+            record_trace(P, N, ks, gi, x, Model<KIND>::NV);
+            if (mon_on<MON>(P)) monitor_state(P, N, ks, i, x, Model<KIND>::NV, sp);
+            if (sp && plastic) note_post_spike(P, N, i, ks);
+        }
+        compact_spikes(P, N, ks, i, sp, false);
+        if (push_inv_dt > 0.0) warp_push<SMALL ? 4 : 1>(P, N, ks, i, sp, push_inv_dt);
+    }
+}
+
+// Steps k .. k+nsteps-1 of one tile, the state in registers between them.
 // push_inv_dt > 0: also fan out the spikes (1 / step, for arrival_step).
+// SMALL: registers are not bounded and a warp keeps more accesses of a fan-out in
+// flight (populations that fit the SMs all the same, see eb_update.cu).
 // HH under BDF holds the Newton state (Jacobian, inverse, history) in about 120
 // registers, which leaves 2 blocks per SM; bounded to 3 blocks (80 registers, a
 // 44-byte spill) a 100k-neuron population fits one wave and its steps take a
@@ -494,10 +752,11 @@ constexpr int narrow_min_blocks(int kind, int integ) {
     return (kind == KIND_HH && integ == INTEG_BDF) ? 3 : (kind != KIND_HH && integ != INTEG_BDF) ? 6 : 0;
 }
 
-template <int KIND, int INTEG, int EN, int MON>
-__global__ void __launch_bounds__(kNarrowTile, narrow_min_blocks(KIND, INTEG)) k_update_narrow(PopDev P, NetDev N, int rel, int nsteps,
+template <int KIND, int INTEG, int EN, int MON, bool SMALL>
+__global__ void __launch_bounds__(kNarrowBlock, SMALL ? 1 : narrow_min_blocks(KIND, INTEG) * (kNarrowTile / kNarrowBlock)) k_update_narrow(PopDev P, NetDev N, int rel, int nsteps,
                                                                 double push_inv_dt, int npw) {
     const int64_t k = cur_step(N, rel);
+    __shared__ NarrowStage<SMALL || KIND == KIND_HH ? narrow_stage(KIND) : 1> stage[kNarrowBlock / 32];
     const int lane = threadIdx.x & 31;
     const int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * npw + lane;
     const bool active = lane < npw && i < P.n;
@@ -507,7 +766,12 @@ __global__ void __launch_bounds__(kNarrowTile, narrow_min_blocks(KIND, INTEG)) k
         load_state<KIND>(P, i, x);
         ax = load_aux<KIND, INTEG>(P, i);
     }
-    for (int s = 0; s < nsteps; ++s) narrow_step<KIND, INTEG, EN, MON>(P, N, k + s, i, active, x, ax, false, push_inv_dt);
+    if constexpr (SMALL || KIND == KIND_HH) {
+        narrow_window<KIND, INTEG, EN, MON, SMALL>(P, N, k, i, active, x, ax, nsteps, push_inv_dt, stage[threadIdx.x >> 5]);
+    } else {
+        for (int s = 0; s < nsteps; ++s)
+            narrow_step<KIND, INTEG, EN, MON>(P, N, k + s, i, active, x, ax, false, push_inv_dt);
+    }
     if (active) {
         store_state<KIND>(P, i, x);
         store_aux<KIND, INTEG>(P, i, ax);
@@ -536,9 +800,6 @@ constexpr int kWideSmem = 1024;
 constexpr int kRankSort = 256;
 static_assert(kRankSort <= kWideThreads && kWideThreads <= kNarrowTile, "wide blocks rank with one thread per arrival");
 
-// Steps of one launch (the runtime's window length).
-constexpr int kMaxWindow = 8;
-
 struct WideSmem {
     int spiked;                         // the block's neuron spiked this step (fused fan-out)
     int ring_ok;                        // ring, ring_f and ring_n hold the neuron's ring
@@ -561,20 +822,6 @@ struct WideSmem {
     float sw[kWideSmem];
     uint8_t sty[kWideSmem];
 };
-
-// Asynchronous global -> shared copies (cp.async): the block copies the next
-// step's arrivals while it works on this one; the copies complete at
-// cp_async_wait_all, before the next step's first barrier.
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Copy step k's arrival count and its first n records (n <= the neuron's bucket
 // capacity) of neuron gi into S.next_c / S.next_rec.  Only for a step whose

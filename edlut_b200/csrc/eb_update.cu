@@ -18,6 +18,10 @@ static int narrow_npw(int64_t n) { return (int)std::min<int64_t>(32, std::max<in
 // blocks of 256; 100,000: 33.4, 32.4).
 static int narrow_tile(int npw) { return npw < 32 ? 32 : 64; }
 
+// Populations that fit the SMs at the register count the unbounded update needs
+// (16 warps an SM at up to 128 registers, HH 12 at 168).
+static int64_t narrow_few(int kind) { return 148 * 32 * (kind == KIND_HH ? 12 : 16); }
+
 template <int KIND, int INTEG>
 void launch_update_t(const PopDev &P, const NetDev &N, int rel, int nsteps, double push_inv_dt, cudaStream_t st) {
     if (P.wide) {
@@ -31,10 +35,12 @@ void launch_update_t(const PopDev &P, const NetDev &N, int rel, int nsteps, doub
         // monitored population takes the generic kernel with the monitor hooks
         const int npw = narrow_npw(P.n), tile = narrow_tile(npw), per = tile / 32 * npw;
         const int blocks = (int)((P.n + per - 1) / per);
-        if (P.mon) k_update_narrow<KIND, INTEG, -1, 1><<<blocks, tile, 0, st>>>(P, N, rel, nsteps, push_inv_dt, npw);
-        else if (P.en == 1) k_update_narrow<KIND, INTEG, 1, 0><<<blocks, tile, 0, st>>>(P, N, rel, nsteps, push_inv_dt, npw);
-        else if (P.en == 3) k_update_narrow<KIND, INTEG, 3, 0><<<blocks, tile, 0, st>>>(P, N, rel, nsteps, push_inv_dt, npw);
-        else k_update_narrow<KIND, INTEG, -1, 0><<<blocks, tile, 0, st>>>(P, N, rel, nsteps, push_inv_dt, npw);
+        auto launch = [&](auto fn) { fn<<<blocks, tile, 0, st>>>(P, N, rel, nsteps, push_inv_dt, npw); };
+        const bool small = P.n <= narrow_few(KIND);
+        if (P.mon) launch(k_update_narrow<KIND, INTEG, -1, 1, true>);
+        else if (P.en == 1) small ? launch(k_update_narrow<KIND, INTEG, 1, 0, true>) : launch(k_update_narrow<KIND, INTEG, 1, 0, false>);
+        else if (P.en == 3) small ? launch(k_update_narrow<KIND, INTEG, 3, 0, true>) : launch(k_update_narrow<KIND, INTEG, 3, 0, false>);
+        else launch(k_update_narrow<KIND, INTEG, -1, 0, false>);
     }
 }
 

@@ -8,25 +8,30 @@
 // every neuron with one delay and static weights; Euler, RK2 or RK4.
 //
 // One CTA owns one network for a chunk of steps (a persistent grid takes networks
-// from an atomic queue, largest first, so uneven sizes balance).  Per step k:
+// from an atomic queue, largest first, so uneven sizes balance).  When there are
+// fewer networks than half the SMs, a cluster of 2, 4 or 8 CTAs owns one, each CTA a
+// tile of its neurons.  Per step k:
 //   1. deliveries: the source steps j whose spikes arrive at step k (one or two;
 //      a host table, because the arrival step of t_j + d flips with the rounding
-//      of the double step times) and the input spikes arriving in the step are
-//      listed in the reference's delivery order -- arrival time, then synapse
-//      order (source, target) -- by thread 0 from the spike bitmasks of the
-//      delay ring held in shared memory.  Every thread loads a batch of the
-//      listed sources' synapses (target, weight) at once, then the batch is
-//      applied one source at a time with a barrier in between: targets of one
-//      source are distinct, so each target receives its additions in list order
-//      without atomics (src/spike/PropagatedSpikeGroup.cpp:112-149);
-//   2. update: each thread advances neurons tid, tid + blockDim, ... (the whole
-//      state -- V, refractory counter, gE, gI -- of the network lives in shared
-//      memory for the chunk) with the model/integrator arithmetic of
-//      the plain path, with the refractory test precomputed per network as step
-//      counts (src/neuron_model/LIFTimeDrivenModel.cpp:160-242);
-//   3. spikes: one warp ballot per 32 neurons is the bitmask word of the step's
-//      ring slot (plus a summary bit per non-zero word); spiking lanes append
-//      their neuron to the network's record.
+//      of the double step times) and the input spikes arriving in the step, listed
+//      in the reference's delivery order -- arrival time, then synapse order (source,
+//      target) -- by one warp from the spike bitmasks of the delay ring in shared
+//      memory.  A spike is needed `lag` steps later, so the steps of a window of up to
+//      8 are listed at its start, a warp each, and the listed rows prefetched into L2.
+//      Every thread loads a batch of the listed sources' synapses (target, weight) at
+//      once, then the batch is applied one source at a time with a barrier in between:
+//      targets of one source are distinct, so each target receives its additions in
+//      list order without atomics (src/spike/PropagatedSpikeGroup.cpp:112-149);
+//   2. update: each thread advances neurons tid, tid + blockDim, ... of its tile (the
+//      state -- V, refractory counter, gE, gI -- lives in shared memory for the chunk)
+//      with the model/integrator arithmetic of the plain path, with the refractory
+//      test precomputed per network as step counts
+//      (src/neuron_model/LIFTimeDrivenModel.cpp:160-242);
+//      (steps without deliveries follow the one before in registers, without a barrier);
+//   3. spikes: one warp ballot per 32 neurons is the bitmask word of the step's ring
+//      slot, stored into the ring of every CTA of the network.  The CTAs of a cluster
+//      meet once per window; the first one then appends the window's spikes to the
+//      network's record.
 // So each network's spikes equal a solo run of the same network on the plain
 // path.  Connectivity and weights come from a counter-based hash of (seed,
 // network, source, target), generated on the device at build time.
@@ -120,31 +125,31 @@ __global__ void k_sweep_fill(const SweepNet *nets, const uint32_t *optr, uint64_
 
 // --------------------------------------------------------------- neuron update --
 // One integration step, operation for operation the plain path's integrate<LIF, INTEG>.
-template <int INTEG>
+template <int INTEG, int EN>
 __device__ __forceinline__ void sw_integrate(const SweepLif &L, float dt, float &V, float &gE, float &gI, int cls, float f) {
     if (INTEG == INTEG_EULER) {
-        const float k1 = sw_deriv(L, V, gE, gI, cls, f);
+        const float k1 = sw_deriv<EN>(L, V, gE, gI, cls, f);
         V += dt * k1;
-        sw_decay(L, gE, gI);
+        sw_decay<EN>(L, gE, gI);
     } else if (INTEG == INTEG_RK2) {
-        const float k1 = sw_deriv(L, V, gE, gI, cls, f);
+        const float k1 = sw_deriv<EN>(L, V, gE, gI, cls, f);
         V += k1 * dt;
-        sw_decay(L, gE, gI);
-        const float k2 = sw_deriv(L, V, gE, gI, cls, f);
+        sw_decay<EN>(L, gE, gI);
+        const float k2 = sw_deriv<EN>(L, V, gE, gI, cls, f);
         V += (-k1 + k2) * dt * 0.5f;
     } else {
         const float h05 = dt * 0.5f;
         const float h016 = dt * 0.166666666667f;
-        const float k1 = sw_deriv(L, V, gE, gI, cls, f);
+        const float k1 = sw_deriv<EN>(L, V, gE, gI, cls, f);
         float a = V + k1 * h05;
         float aE = gE, aI = gI;
-        sw_decay(L, aE, aI);
-        const float k2 = sw_deriv(L, a, aE, aI, cls, f);
+        sw_decay<EN>(L, aE, aI);
+        const float k2 = sw_deriv<EN>(L, a, aE, aI, cls, f);
         a = V + k2 * h05;
-        const float k3 = sw_deriv(L, a, aE, aI, cls, f);
+        const float k3 = sw_deriv<EN>(L, a, aE, aI, cls, f);
         a = V + k3 * dt;
-        sw_decay(L, aE, aI);
-        const float k4 = sw_deriv(L, a, aE, aI, cls, f);
+        sw_decay<EN>(L, aE, aI);
+        const float k4 = sw_deriv<EN>(L, a, aE, aI, cls, f);
         V += (k1 + 2.0f * (k2 + k3) + k4) * h016;
         gE = aE;
         gI = aI;
@@ -161,294 +166,422 @@ __device__ __forceinline__ int list_rank(const int32_t *off, int S, int e) {
     return lo;
 }
 
+// First synapse of every source in each of `ctas` tiles of its network's neurons (one
+// thread per source and tile boundary, bisection in the source's ascending targets).
+__global__ void k_sweep_tiles(SweepDev G, int ctas, uint32_t *tptr) {
+    const SweepNet &S = G.nets[blockIdx.y];
+    const int tile = (S.wn + ctas - 1) / ctas * 32;
+    const int64_t items = (int64_t)(S.n + S.n_in) * (ctas + 1);
+    const uint16_t *tg = G.tgt + S.syn_off;
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < items; x += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t s = x / (ctas + 1);
+        const int first = (int)(x - s * (ctas + 1)) * tile;
+        uint32_t lo = G.optr[S.src_off + s], hi = G.optr[S.src_off + s + 1];
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if ((int)tg[mid] < first) lo = mid + 1; else hi = mid;
+        }
+        tptr[S.src_off * (ctas + 1) + x] = lo;
+    }
+}
+
+// One step's sources in delivery order, with the synapses they have in the CTA's tile.
+struct SweepList {
+    int32_t *src, *off;     // [cap], [cap + 1]: source, running total of synapses
+    uint32_t *base;         // [cap]: its first synapse
+};
+
 struct SweepSmem {
-    float *V, *gE, *gI;
-    int32_t *rf;            // refractory counters
-    uint32_t *ring, *sum;   // [R][wc], [R][swc]
-    int32_t *src, *off;     // [kListCap], [kListCap + 1]
-    uint32_t *base;         // [kListCap]
+    float4 *x;              // [tile] V, gE, gI, refractory counter (integer bits)
+    uint32_t *ring;         // [R][wc] spike bitmasks of the whole network
+    int32_t *lists;         // the lists of a window's steps
+    int cap;
+    __device__ SweepList list(int s) const {
+        int32_t *p = lists + s * (3 * cap + 1);
+        return SweepList{p, p + cap, reinterpret_cast<uint32_t *>(p + 2 * cap + 1)};
+    }
 };
 
-// Thread 0's delivery-list generator for one step: input spikes of phase 0, the
-// spikes of the first arriving source step, inputs of phase 1, ... in order.
-struct ListGen {
-    int g, G, lo, part, a, q, slot;
-    uint32_t sm, m;
-    int64_t cur;      // input cursor
-    int32_t nkey;     // key of input cur (INT_MAX when exhausted)
-    int32_t nsrc;
+size_t sweep_smem_bytes(int tile, int R, int wc, int window, int cap) {
+    return 16 * (size_t)tile + sizeof(uint32_t) * (size_t)R * wc + window * sizeof(int32_t) * (3 * (size_t)cap + 1);
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Barrier of every thread of the cluster, ordering shared-memory stores across it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Store v at the place of p in the shared memory of the cluster's CTA `rank`.
+__device__ __forceinline__ void cluster_store(uint32_t *p, uint32_t rank, uint32_t v) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(rank));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ int warp_incl_scan(int v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    return v;
+}
+
+// First input spike at or after `cur` whose key reaches `key` (one warp, 32 at a time).
+__device__ __forceinline__ int64_t seek_input(const SweepDev &G, const SweepNet &S, int64_t cur, int32_t key, int lane) {
+    for (;;) {
+        const bool below = cur + lane < S.n_in_spikes && G.in_key[S.in_off + cur + lane] < key;
+        const int c = __popc(__ballot_sync(0xffffffffu, below));
+        cur += c;
+        if (c < 32) return cur;
+    }
+}
+
+// One warp lists step k's sources, positions [p0, p0 + cap) of the delivery order, into
+// B: per phase the inputs of its key (from input `cur` on), then the spikes of the
+// next arriving source step in neuron order; then their synapse ranges and running
+// totals, and their rows on the way into L2.  Returns the sources of the whole step.
+__device__ __forceinline__ int list_step(const SweepDev &G, const SweepSmem &M, const SweepNet &S, const SweepList &B,
+                                         int64_t cur, int64_t k, int p0, int wc, int tile, int lane) {
+    constexpr unsigned full = 0xffffffffu;
+    const int lo = G.grp_lo[k], groups = G.grp_n[k], cap = M.cap;
+    int pos = 0;
+    for (int g = 0; g <= groups; ++g) {
+        for (;;) {  // inputs of phase g
+            const int64_t q = cur + lane;
+            const bool mine = q < S.n_in_spikes && G.in_key[S.in_off + q] == (int32_t)(k * 4) + g;
+            const int c = __popc(__ballot_sync(full, mine));
+            const int p = pos + lane - p0;
+            if (mine && p >= 0 && p < cap) B.src[p] = S.n + G.in_src[S.in_off + q];
+            pos += c;
+            cur += c;
+            if (c < 32) break;
+        }
+        if (g == groups) break;
+        const uint32_t *row = M.ring + (int)((uint32_t)(lo + g) % (uint32_t)G.R) * wc;
+        for (int a = 0; a < S.wn; a += 32) {
+            if (a % 256 == 0) {  // 8,192 neurons at once: most steps have few spikes or none
+                uint32_t any = 0;
+#pragma unroll
+                for (int u = 0; u < 256; u += 32) any |= a + u + lane < S.wn ? row[a + u + lane] : 0u;
+                if (!__any_sync(full, any != 0)) { a += 256 - 32; continue; }
+            }
+            uint32_t w = a + lane < S.wn ? row[a + lane] : 0u;
+            if (!__any_sync(full, w != 0)) continue;
+            const int c = __popc(w);
+            const int incl = warp_incl_scan(c, lane);
+            int p = pos + incl - c - p0;
+            while (w) {
+                const int b = __ffs(w) - 1;
+                w &= w - 1u;
+                if (p >= 0 && p < cap) B.src[p] = (a + lane) * 32 + b;
+                ++p;
+            }
+            pos += __shfl_sync(full, incl, 31);
+        }
+    }
+    __syncwarp();
+    const int cnt = min(pos - p0, cap);
+    int carry = 0;
+    for (int b = 0; b < cnt; b += 32) {
+        const int x = b + lane;
+        uint32_t first = 0;
+        int fan = 0;
+        if (x < cnt) {
+            const uint32_t *t = G.tptr + (S.src_off + B.src[x]) * G.tstride + tile;
+            first = __ldg(t);
+            fan = (int)(__ldg(t + 1) - first);
+        }
+        const int incl = warp_incl_scan(fan, lane);
+        if (x < cnt) {
+            B.off[x] = carry + incl - fan;
+            B.base[x] = first;
+            if (fan > 0) {  // whole 16-byte units around the row
+                const uint64_t t = (uint64_t)(G.tgt + S.syn_off + first), w = (uint64_t)(G.w + S.syn_off + first);
+                const uint64_t t0 = t & ~15ull, w0 = w & ~15ull;
+                const uint32_t nt = (uint32_t)((t + 2ull * fan - t0 + 15) & ~15ull);
+                const uint32_t nw = (uint32_t)((w + 4ull * fan - w0 + 15) & ~15ull);
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(t0), "r"(nt) : "memory");
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w0), "r"(nw) : "memory");
+            }
+        }
+        carry += __shfl_sync(full, incl, 31);
+    }
+    if (lane == 0 && cnt > 0) B.off[cnt] = carry;
+    return pos;
+}
+
+// Neurons whose V this thread records after every step: it owns up to two observed
+// ones (i: index in the tile, m: observed slot).
+struct SweepObs {
+    int i0, m0, i1, m1;
 };
 
-template <int INTEG, bool TRAJ>
-__device__ void sweep_network(const SweepDev &G, const SweepSmem &M, const SweepNet &S, const SweepLif &L, int net,
-                              int64_t k0, int nsteps, int wc, int swc, int64_t traj_k0) {
-    __shared__ int s_S, s_more;
-    __shared__ uint32_t s_rec_n;
+// The CTA's update of its tile at steps k .. k + run - 1, none of which but the first
+// has deliveries: integrate, spike test, bitmask words into the steps' ring slots of
+// every CTA of the network.  The sweep is bound by the instructions of this loop: a
+// neuron's state is one 16-byte word of shared memory, loaded once for the steps, and
+// the refractory class selects (no branches).
+template <int INTEG, bool TRAJ, int EN, bool CL>
+__device__ __forceinline__ void sweep_update(const SweepDev &G, const SweepSmem &M, const SweepLif &L, const SweepLif &Ls,
+                                             const SweepObs &O, int nl, int first, int run, int slot0, int wc, int64_t x0,
+                                             float *trace) {
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, ctas = G.ctas;
+    const float dt = G.dt_ms;
+    const int wrap = G.R * wc;
+    for (int i = tid; i - lane < nl; i += nt) {
+        const bool valid = i < nl;
+        float4 x = M.x[valid ? i : 0];
+        int rr = __float_as_int(x.w);
+        int word = slot0 * wc + ((first + i) >> 5);
+        for (int t = 0; t < run; ++t) {
+            const bool late = (unsigned)rr < (unsigned)L.r_free;  // refractory, and not the -1 of no spike yet
+            const bool frozen = late && rr < L.r_frac0, part = late && !frozen;
+            const int fi = part ? rr - L.r_frac0 : 0;
+            float f = 1.0f;
+            if (part) f = Ls.frac[fi];
+            if (TRAJ && valid) {
+                const int64_t o = x0 + t * G.n_total + i;
+                G.tV[o] = x.x;
+                G.tE[o] = x.y;
+                G.tI[o] = x.z;
+            }
+            sw_integrate<INTEG, EN>(L, dt, x.x, x.y, x.z, frozen ? 1 : 2, f);
+            if (rr >= 0) rr++;
+            const bool sp = x.x > L.v_thr;
+            x.x = sp ? L.e_leak : x.x;
+            rr = sp ? 0 : rr;
+            if (TRAJ && valid)
+                G.tcode[x0 + t * G.n_total + i] = (uint8_t)((frozen ? 1 : part ? 2 : 0) | (fi << 2) | (sp ? kCodeSpike : 0));
+            if (x.x != x.x) { x.x = L.e_leak; x.y = 0.0f; x.z = 0.0f; }
+            if (i == O.i0) trace[t * G.n_obs + O.m0] = x.x;
+            if (i == O.i1) trace[t * G.n_obs + O.m1] = x.x;
+            const unsigned m = __ballot_sync(0xffffffffu, sp && valid);
+            if (CL) { if (lane < ctas) cluster_store(M.ring + word, lane, m); }
+            else if (lane == 0) M.ring[word] = m;
+            word += wc;
+            if (word >= wrap) word -= wrap;
+        }
+        x.w = __int_as_float(rr);
+        if (valid) M.x[i] = x;
+    }
+}
+
+// Append the spikes of steps k_first .. k_first + len - 1 to the network's record, in
+// (step, neuron) order, from the ring's bitmasks (one CTA, whole block).
+__device__ __forceinline__ void drain_window(const SweepDev &G, const SweepSmem &M, const SweepNet &S, int net, int64_t k_first,
+                                             int len, int wc, uint32_t *s_cnt, uint32_t &rec_n) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    for (int s = warp; s < len; s += nwarps) {
+        const uint32_t *row = M.ring + (int)((uint32_t)(k_first + s) % (uint32_t)G.R) * wc;
+        int c = 0;
+        for (int a = lane; a < S.wn; a += 32) c += __popc(row[a]);
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) s_cnt[s] = (uint32_t)c;
+    }
+    __syncthreads();
+    uint32_t at = rec_n;
+    for (int s = 0; s < len; ++s) {
+        const uint32_t c = s_cnt[s];
+        if ((s & (nwarps - 1)) == warp && c) {
+            const uint32_t *row = M.ring + (int)((uint32_t)(k_first + s) % (uint32_t)G.R) * wc;
+            uint32_t pos = at;
+            for (int a = 0; a < S.wn; a += 32) {
+                uint32_t w = a + lane < S.wn ? row[a + lane] : 0u;
+                if (!__any_sync(0xffffffffu, w != 0)) continue;
+                const int n = __popc(w);
+                const int incl = warp_incl_scan(n, lane);
+                uint32_t x = pos + (uint32_t)(incl - n);
+                while (w) {
+                    const int b = __ffs(w) - 1;
+                    w &= w - 1u;
+                    if ((int64_t)x < S.rec_cap) G.rec[S.rec_off + x] = (uint16_t)((a + lane) * 32 + b);
+                    else atomicOr(G.flags, FLAG_RECORD_OVERFLOW);
+                    ++x;
+                }
+                pos += (uint32_t)__shfl_sync(0xffffffffu, incl, 31);
+            }
+        }
+        at += c;
+        if (threadIdx.x == 0) G.rec_end[(int64_t)net * G.steps_max + (k_first + s - 1)] = (int32_t)at;
+    }
+    rec_n = at;
+}
+
+template <int INTEG, bool TRAJ, bool CL>
+__device__ void sweep_network(const SweepDev &G, const SweepSmem &M, const SweepNet &S, const SweepLif &Ls, int net, int tile,
+                              int64_t k0, int nsteps, int wc, int64_t traj_k0) {
+    __shared__ int s_cnt[kSweepWindow];   // sources of each step of the window
+    __shared__ uint32_t s_win[kSweepWindow];
     const int n = S.n, n_exc = S.n_exc;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    const int nj = (n + nt - 1) / nt;
-    const int R = G.R;
-    const int wn = S.wn, swn = (wn + 31) >> 5;
-    const int64_t so = S.state_off;
-    const uint32_t *optr = G.optr + S.src_off;
+    const int R = G.R, C = G.ctas, wn = S.wn, cap = M.cap;
+    const int first = (wn + C - 1) / C * 32 * tile;               // the tile's neurons
+    const int nl = max(0, min(n - first, (wn + C - 1) / C * 32));
+    const int64_t so = S.state_off + first;
     const uint16_t *tg = G.tgt + S.syn_off;
     const float *ww = G.w + S.syn_off;
-    const float dt = G.dt_ms;
+    const SweepLif L = Ls;  // in registers; the fractions are indexed in shared memory
 
-    for (int i = tid; i < n; i += nt) {
-        M.V[i] = G.V[so + i];
-        M.rf[i] = G.refr[so + i];
-        M.gE[i] = G.gE[so + i];
-        M.gI[i] = G.gI[so + i];
-    }
+    for (int i = tid; i < nl; i += nt)
+        M.x[i] = make_float4(G.V[so + i], G.gE[so + i], G.gI[so + i], __int_as_float(G.refr[so + i]));
     for (int x = tid; x < R * wc; x += nt) {
         const int slot = x / wc, q = x - slot * wc;
         M.ring[x] = q < wn ? G.ring[S.ring_off + (int64_t)slot * wn + q] : 0u;
     }
-    for (int x = tid; x < R * swc; x += nt) {
-        const int slot = x / swc, a = x - slot * swc;
-        M.sum[x] = a < swn ? G.rsum[S.sum_off + (int64_t)slot * swn + a] : 0u;
-    }
-    ListGen gen;
+    // observed neurons: written by their owners while nobody owns more than two, else
+    // read by the block after every step
+    SweepObs O{-1, 0, -1, 0};
+    bool many = G.n_obs > kOwnObs;
+    const int32_t *obs = G.obs + (int64_t)net * G.n_obs;
+    if (!many)
+        for (int m = 0; m < G.n_obs; ++m) {
+            const int i = obs[m] - first;
+            if (i < 0 || i >= nl || i % nt != tid) continue;
+            many = many || O.i1 >= 0;
+            if (O.i0 < 0) { O.i0 = i; O.m0 = m; }
+            else { O.i1 = i; O.m1 = m; }
+        }
+    many = __syncthreads_or(many);
+    if (many) O.i0 = O.i1 = -1;
     unsigned long long events = 0;
-    int nx_lo = 0, nx_G = 0;
-    if (tid == 0) {
-        s_rec_n = G.rec_cnt[net];
-        gen.cur = G.in_cursor[net];
-        gen.nkey = INT_MAX;
-        gen.nsrc = 0;
-        if (gen.cur < S.n_in_spikes) { gen.nkey = G.in_key[S.in_off + gen.cur]; gen.nsrc = G.in_src[S.in_off + gen.cur]; }
-        nx_lo = G.grp_lo[k0 + 1];
-        nx_G = G.grp_n[k0 + 1];
-    }
-    __syncthreads();
+    uint32_t rec_n = tile == 0 ? G.rec_cnt[net] : 0u;
+    int64_t cur = G.in_cursor[net];  // this warp's place in the input spikes
+    if (CL) cluster_sync();  // every ring is loaded before another CTA's spikes reach it
 
-    for (int r = 0; r < nsteps; ++r) {
-        const int64_t k = k0 + r + 1;
-        // ---------------------------------------------------- 1. deliveries
-        if (tid == 0) {
-            if (r > 0) G.rec_end[(int64_t)net * G.steps_max + (k - 2)] = (int32_t)s_rec_n;
-            gen.g = 0;
-            gen.G = nx_G;
-            gen.lo = nx_lo;
-            gen.part = 0;
-            if (k + 1 <= G.steps_max) { nx_lo = G.grp_lo[k + 1]; nx_G = G.grp_n[k + 1]; }
-        }
-        const int32_t key0 = (int32_t)(k * 4);
-        for (;;) {
-            if (tid == 0) {
-                int cnt = 0;
-                bool done = false;
-                while (cnt < kListCap) {
-                    if (gen.part == 0) {
-                        if (gen.nkey == key0 + gen.g) {
-                            M.src[cnt++] = n + gen.nsrc;
-                            ++gen.cur;
-                            gen.nkey = INT_MAX;
-                            if (gen.cur < S.n_in_spikes) {
-                                gen.nkey = G.in_key[S.in_off + gen.cur];
-                                gen.nsrc = G.in_src[S.in_off + gen.cur];
-                            }
-                            continue;
-                        }
-                        if (gen.g >= gen.G) { done = true; break; }
-                        gen.part = 1;
-                        gen.slot = (int)((gen.lo + gen.g) % R);
-                        gen.a = 0;
-                        gen.sm = M.sum[gen.slot * swc];
-                        gen.m = 0;
-                        continue;
-                    }
-                    if (gen.m) {
-                        const int b = __ffs(gen.m) - 1;
-                        gen.m &= gen.m - 1u;
-                        M.src[cnt++] = gen.q * 32 + b;
-                        continue;
-                    }
-                    if (gen.sm) {
-                        const int b = __ffs(gen.sm) - 1;
-                        gen.sm &= gen.sm - 1u;
-                        gen.q = gen.a * 32 + b;
-                        gen.m = M.ring[gen.slot * wc + gen.q];
-                        continue;
-                    }
-                    if (++gen.a < swc) { gen.sm = M.sum[gen.slot * swc + gen.a]; continue; }
-                    gen.part = 0;
-                    ++gen.g;
-                }
-                s_S = cnt;
-                s_more = done ? 0 : 1;
-            }
-            __syncthreads();
-            const int Sn = s_S, more = s_more;
-            if (Sn > 0) {
-                if (warp == 0) {
-                    int carry = 0;
-                    for (int b = 0; b < Sn; b += 32) {
-                        const int x = b + lane;
-                        uint32_t lo = 0;
-                        int fan = 0;
-                        if (x < Sn) {
-                            const int s = M.src[x];
-                            lo = __ldg(optr + s);
-                            fan = (int)(__ldg(optr + s + 1) - lo);
-                        }
-                        int incl = fan;
-#pragma unroll
-                        for (int o = 1; o < 32; o <<= 1) {
-                            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                            if (lane >= o) incl += u;
-                        }
-                        if (x < Sn) { M.off[x] = carry + incl - fan; M.base[x] = lo; }
-                        carry += __shfl_sync(0xffffffffu, incl, 31);
-                    }
-                    if (lane == 0) M.off[Sn] = carry;
-                }
-                __syncthreads();
-                const int total = M.off[Sn];
-                for (int e0 = 0; e0 < total; e0 += kBatch * nt) {
-                    uint16_t tq[kBatch];
-                    float wq[kBatch];
-                    int rk[kBatch];
-                    bool inh[kBatch];
-#pragma unroll
-                    for (int q = 0; q < kBatch; ++q) {
-                        const int e = e0 + q * nt + tid;
-                        rk[q] = -1;
-                        tq[q] = 0;
-                        wq[q] = 0.0f;
-                        inh[q] = false;
-                        if (e < total) {
-                            const int a = list_rank(M.off, Sn, e);
-                            const uint32_t o = M.base[a] + (uint32_t)(e - M.off[a]);
-                            tq[q] = __ldg(tg + o);
-                            wq[q] = __ldg(ww + o);
-                            const int s = M.src[a];
-                            inh[q] = s >= n_exc && s < n;
-                            rk[q] = a;
-                        }
-                    }
-                    const int r_lo = list_rank(M.off, Sn, e0);
-                    const int r_hi = list_rank(M.off, Sn, min(e0 + kBatch * nt, total) - 1);
-                    for (int a = r_lo; a <= r_hi; ++a) {
-#pragma unroll
-                        for (int q = 0; q < kBatch; ++q)
-                            if (rk[q] == a) {
-                                float *g = inh[q] ? M.gI : M.gE;
-                                g[tq[q]] += wq[q];
-                            }
-                        __syncthreads();
-                    }
-                }
-                if (tid == 0) events += (unsigned long long)total;
-            }
-            if (!more) break;
-            __syncthreads();
-        }
-        // -------------------------------------------------- 2. update, 3. spikes
-        const int slot = (int)(k % R);
-        for (int j = 0; j < nj; ++j) {
-            {
-                const int i = tid + j * nt;
-                bool sp = false;
-                if (i < n) {
-                    float v = M.V[i], gE = M.gE[i], gI = M.gI[i];
-                    int rr = M.rf[i];
-                    int cls = 0, fi = 0;
-                    float f = 1.0f;
-                    if (rr >= 0 && rr < L.r_free) {
-                        if (rr >= L.r_frac0) { cls = 2; fi = rr - L.r_frac0; f = L.frac[fi]; }
-                        else cls = 1;
-                    }
-                    if (TRAJ) {
-                        const int64_t x = (k - traj_k0 - 1) * G.n_total + so + i;
-                        G.tV[x] = v;
-                        G.tE[x] = gE;
-                        G.tI[x] = gI;
-                    }
-                    sw_integrate<INTEG>(L, dt, v, gE, gI, cls, f);
-                    if (rr >= 0) rr++;
-                    if (v > L.v_thr) { v = L.e_leak; sp = true; rr = 0; }
-                    if (TRAJ) G.tcode[(k - traj_k0 - 1) * G.n_total + so + i] = (uint8_t)(cls | (fi << 2) | (sp ? kCodeSpike : 0));
-                    if (v != v) { v = L.e_leak; gE = 0.0f; gI = 0.0f; }
-                    M.V[i] = v;
-                    M.rf[i] = rr;
-                    M.gE[i] = gE;
-                    M.gI[i] = gI;
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, sp);
-                const int q = j * nwarps + warp;
-                uint32_t base = 0;
-                if (lane == 0) {
-                    M.ring[slot * wc + q] = m;
-                    if (m) {
-                        atomicOr(&M.sum[slot * swc + (q >> 5)], 1u << (q & 31));
-                        base = atomicAdd(&s_rec_n, (uint32_t)__popc(m));
-                    }
-                }
-                if (m) {
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if (sp) {
-                        const uint32_t x = base + __popc(m & ((1u << lane) - 1u));
-                        if ((int64_t)x < S.rec_cap) G.rec[S.rec_off + x] = (uint16_t)i;
-                        else atomicOr(G.flags, FLAG_RECORD_OVERFLOW);
-                    }
-                }
-            }
-        }
-        if (tid == 0) {
-            // the slot written at step k+1 starts with an empty summary
-            const int ns = (int)((k + 1) % R);
-            for (int a = 0; a < swc; ++a) M.sum[ns * swc + a] = 0u;
+    for (int w0 = 0; w0 < nsteps; w0 += G.window) {
+        const int64_t kw = k0 + w0 + 1;  // the window's first step
+        const int len = min(G.window, nsteps - w0);
+        for (int s = warp; s < len; s += nwarps) {
+            cur = seek_input(G, S, cur, (int32_t)((kw + s) * 4), lane);
+            const int c = list_step(G, M, S, M.list(s), cur, kw + s, 0, wc, tile, lane);
+            if (lane == 0) s_cnt[s] = c;
         }
         __syncthreads();
-        // observed membrane potentials after step k
-        for (int m = tid; m < G.n_obs; m += nt)
-            G.trace[((int64_t)net * G.steps_max + (k - 1)) * G.n_obs + m] = M.V[G.obs[(int64_t)net * G.n_obs + m]];
+        for (int s = 0; s < len;) {
+            const int64_t k = kw + s;
+            const int sources = s_cnt[s];
+            // ------------------------------------------------ 1. deliveries
+            if (sources > 0) {
+                if (s > 0) __syncthreads();  // the last update is done
+                const SweepList B = M.list(s);
+                for (int p0 = 0;; p0 += cap) {
+                    const int Sn = min(sources - p0, cap);
+                    const int total = B.off[Sn];
+                    for (int e0 = 0; e0 < total; e0 += kBatch * nt) {
+                        uint16_t tq[kBatch];
+                        float wq[kBatch];
+                        int rk[kBatch];
+                        bool inh[kBatch];
+#pragma unroll
+                        for (int q = 0; q < kBatch; ++q) {
+                            const int e = e0 + q * nt + tid;
+                            rk[q] = -1;
+                            tq[q] = 0;
+                            wq[q] = 0.0f;
+                            inh[q] = false;
+                            if (e < total) {
+                                const int a = list_rank(B.off, Sn, e);
+                                const uint32_t o = B.base[a] + (uint32_t)(e - B.off[a]);
+                                tq[q] = __ldg(tg + o);
+                                wq[q] = __ldg(ww + o);
+                                const int x = B.src[a];
+                                inh[q] = x >= n_exc && x < n;
+                                rk[q] = a;
+                            }
+                        }
+                        const int r_lo = list_rank(B.off, Sn, e0);
+                        const int r_hi = list_rank(B.off, Sn, min(e0 + kBatch * nt, total) - 1);
+                        for (int a = r_lo; a <= r_hi; ++a) {
+#pragma unroll
+                            for (int q = 0; q < kBatch; ++q)
+                                if (rk[q] == a) {
+                                    float4 &x = M.x[tq[q] - first];
+                                    if (inh[q]) x.z += wq[q];
+                                    else x.y += wq[q];
+                                }
+                            __syncthreads();
+                        }
+                    }
+                    if (tid == 0) events += (unsigned long long)total;
+                    if (p0 + cap >= sources) break;
+                    __syncthreads();  // every thread is done with this pass's list
+                    if (warp == 0) {
+                        const int64_t c0 = seek_input(G, S, G.in_cursor[net], (int32_t)(k * 4), lane);
+                        list_step(G, M, S, B, c0, k, p0 + cap, wc, tile, lane);
+                    }
+                    __syncthreads();
+                }
+            }
+            // ---------------------------------------------- 2. update, 3. spikes
+            int run = 1;
+            if (!many)
+                while (s + run < len && s_cnt[s + run] == 0) ++run;
+            const int slot = (int)((uint32_t)k % (uint32_t)R);
+            const int64_t x0 = TRAJ ? (k - traj_k0 - 1) * G.n_total + so : 0;
+            float *trace = G.trace + ((int64_t)net * G.steps_max + (k - 1)) * G.n_obs;
+            if (L.en == 3) sweep_update<INTEG, TRAJ, 3, CL>(G, M, L, Ls, O, nl, first, run, slot, wc, x0, trace);
+            else sweep_update<INTEG, TRAJ, -1, CL>(G, M, L, Ls, O, nl, first, run, slot, wc, x0, trace);
+            if (many) {
+                __syncthreads();
+                for (int m = tid; m < G.n_obs; m += nt) {
+                    const int i = obs[m] - first;
+                    if (i >= 0 && i < nl) trace[m] = M.x[i].x;
+                }
+                __syncthreads();  // read before the next step writes them
+            }
+            s += run;
+        }
+        if (CL) cluster_sync();
+        else __syncthreads();
+        if (tile == 0) drain_window(G, M, S, net, kw, len, wc, s_win, rec_n);
     }
     // save the network's state
-    for (int i = tid; i < n; i += nt) {
-        G.V[so + i] = M.V[i];
-        G.refr[so + i] = M.rf[i];
-        G.gE[so + i] = M.gE[i];
-        G.gI[so + i] = M.gI[i];
+    for (int i = tid; i < nl; i += nt) {
+        const float4 x = M.x[i];
+        G.V[so + i] = x.x;
+        G.refr[so + i] = __float_as_int(x.w);
+        G.gE[so + i] = x.y;
+        G.gI[so + i] = x.z;
     }
-    for (int x = tid; x < R * wn; x += nt) {
-        const int slot = x / wn, q = x - slot * wn;
-        G.ring[S.ring_off + x] = M.ring[slot * wc + q];
-    }
-    for (int x = tid; x < R * swn; x += nt) {
-        const int slot = x / swn, a = x - slot * swn;
-        G.rsum[S.sum_off + x] = M.sum[slot * swc + a];
+    if (CL) cluster_sync();  // every CTA has read the input cursor
+    if (tile == 0) {
+        for (int x = tid; x < R * wn; x += nt) {
+            const int s = x / wn, q = x - s * wn;
+            G.ring[S.ring_off + x] = M.ring[s * wc + q];
+        }
+        if (warp == 0) {
+            cur = seek_input(G, S, cur, (int32_t)((k0 + nsteps + 1) * 4), lane);
+            if (lane == 0) G.in_cursor[net] = cur;
+        }
     }
     if (tid == 0) {
-        if (nsteps > 0) G.rec_end[(int64_t)net * G.steps_max + (k0 + nsteps - 1)] = (int32_t)s_rec_n;
-        G.rec_cnt[net] = s_rec_n;
-        G.in_cursor[net] = gen.cur;
-        G.events[net] += events;
+        if (tile == 0) G.rec_cnt[net] = rec_n;
+        if (CL) atomicAdd(&G.events[net], events);
+        else G.events[net] += events;
     }
     __syncthreads();
 }
 
-template <int INTEG, bool TRAJ>
-__global__ void __launch_bounds__(1024) k_sweep(SweepDev G, int nsteps, int max_n, int wc, int swc, int64_t traj_k0) {
+template <int INTEG, bool TRAJ, bool CL>
+__global__ void __launch_bounds__(1024) k_sweep(SweepDev G, int nsteps, int max_tile, int wc, int64_t traj_k0) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SweepSmem M;
-    M.V = reinterpret_cast<float *>(smem_raw);
-    M.gE = M.V + max_n;
-    M.gI = M.gE + max_n;
-    M.rf = reinterpret_cast<int32_t *>(M.gI + max_n);
-    M.ring = reinterpret_cast<uint32_t *>(M.rf + max_n);
-    M.sum = M.ring + G.R * wc;
-    M.src = reinterpret_cast<int32_t *>(M.sum + G.R * swc);
-    M.off = M.src + kListCap;
-    M.base = reinterpret_cast<uint32_t *>(M.off + kListCap + 1);
+    M.x = reinterpret_cast<float4 *>(smem_raw);
+    M.ring = reinterpret_cast<uint32_t *>(M.x + max_tile);
+    M.lists = reinterpret_cast<int32_t *>(M.ring + G.R * wc);
+    M.cap = G.list_cap;
     __shared__ int s_net;
     __shared__ SweepLif s_L;
     __shared__ SweepNet s_desc;
     const int64_t k0 = *G.step;
+    const int tile = CL ? (int)cluster_rank() : 0;
     for (;;) {
-        if (threadIdx.x == 0) s_net = atomicAdd(G.queue, 1);
+        if (threadIdx.x == 0) s_net = CL ? (int)blockIdx.x / G.ctas : atomicAdd(G.queue, 1);  // CL: a cluster per network
         __syncthreads();
         const int qi = s_net;
         if (qi >= G.n_nets) break;
@@ -461,7 +594,8 @@ __global__ void __launch_bounds__(1024) k_sweep(SweepDev G, int nsteps, int max_
         __syncthreads();
         if (threadIdx.x == 0) s_L = s_desc.L;
         __syncthreads();
-        sweep_network<INTEG, TRAJ>(G, M, s_desc, s_L, net, k0, nsteps, wc, swc, traj_k0);
+        sweep_network<INTEG, TRAJ, CL>(G, M, s_desc, s_L, net, tile, k0, nsteps, wc, traj_k0);
+        if (CL) break;
     }
 }
 
@@ -476,13 +610,19 @@ __global__ void k_sweep_advance(int64_t *step, int *queue, int nsteps) {
 // ------------------------------------------------------------------- host --
 namespace {
 
-using SweepFn = void (*)(SweepDev, int, int, int, int, int64_t);
+using SweepFn = void (*)(SweepDev, int, int, int, int64_t);
 
-SweepFn sweep_fn(int integ, bool traj) {
+template <int INTEG>
+SweepFn sweep_fn_t(bool traj, bool clustered) {
+    if (clustered) return traj ? k_sweep<INTEG, true, true> : k_sweep<INTEG, false, true>;
+    return traj ? k_sweep<INTEG, true, false> : k_sweep<INTEG, false, false>;
+}
+
+SweepFn sweep_fn(int integ, bool traj, bool clustered) {
     switch (integ) {
-    case INTEG_EULER: return traj ? k_sweep<INTEG_EULER, true> : k_sweep<INTEG_EULER, false>;
-    case INTEG_RK2: return traj ? k_sweep<INTEG_RK2, true> : k_sweep<INTEG_RK2, false>;
-    default: return traj ? k_sweep<INTEG_RK4, true> : k_sweep<INTEG_RK4, false>;
+    case INTEG_EULER: return sweep_fn_t<INTEG_EULER>(traj, clustered);
+    case INTEG_RK2: return sweep_fn_t<INTEG_RK2>(traj, clustered);
+    default: return sweep_fn_t<INTEG_RK4>(traj, clustered);
     }
 }
 
@@ -491,8 +631,18 @@ SweepFn sweep_fn(int integ, bool traj) {
 namespace ebsw {
 
 int enqueue_chunk(eb_sweep *h, int nsteps, cudaStream_t st, bool traj, int64_t traj_k0) {
-    SweepFn f = sweep_fn(h->integ, traj);
-    f<<<h->grid, h->block, h->smem, st>>>(h->G, nsteps, h->max_n, h->wc, h->swc, traj_k0);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(h->grid);
+    cfg.blockDim = dim3(h->block);
+    cfg.dynamicSmemBytes = h->smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = h->G.ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = h->G.ctas > 1 ? 1 : 0;
+    SK(cudaLaunchKernelEx(&cfg, sweep_fn(h->integ, traj, h->G.ctas > 1), h->G, nsteps, h->max_tile, h->wc, traj_k0));
     k_sweep_advance<<<1, 1, 0, st>>>(h->G.step, h->G.queue, nsteps);
     SK(cudaGetLastError());
     return EB_OK;
@@ -501,29 +651,29 @@ int enqueue_chunk(eb_sweep *h, int nsteps, cudaStream_t st, bool traj, int64_t t
 // The arrays that make up the dynamic state, in checkpoint order.
 static void state_arrays(eb_sweep *h, void **ptr, size_t *bytes) {
     const size_t nt = (size_t)h->state_n, B = (size_t)h->n_nets;
-    void *p[9] = {h->G.V, h->G.gE, h->G.gI, h->G.refr, h->G.ring, h->G.rsum, h->G.in_cursor, h->G.rec_cnt, h->G.events};
-    size_t b[9] = {4 * nt, 4 * nt, 4 * nt, 4 * nt, 4 * (size_t)h->ring_words, 4 * (size_t)h->sum_words, 8 * B, 4 * B, 8 * B};
-    for (int i = 0; i < 9; ++i) { ptr[i] = p[i]; bytes[i] = (b[i] + 255) / 256 * 256; }
-    for (int i = 0; i < 9; ++i) bytes[i] = b[i] ? bytes[i] : 0;
+    void *p[8] = {h->G.V, h->G.gE, h->G.gI, h->G.refr, h->G.ring, h->G.in_cursor, h->G.rec_cnt, h->G.events};
+    size_t b[8] = {4 * nt, 4 * nt, 4 * nt, 4 * nt, 4 * (size_t)h->ring_words, 8 * B, 4 * B, 8 * B};
+    for (int i = 0; i < 8; ++i) { ptr[i] = p[i]; bytes[i] = (b[i] + 255) / 256 * 256; }
+    for (int i = 0; i < 8; ++i) bytes[i] = b[i] ? bytes[i] : 0;
 }
 
 size_t checkpoint_bytes(eb_sweep *h) {
-    void *p[9];
-    size_t b[9], t = 0;
+    void *p[8];
+    size_t b[8], t = 0;
     state_arrays(h, p, b);
     for (size_t x : b) t += x;
     return t;
 }
 
 int checkpoint_save(eb_sweep *h, int c, cudaStream_t st) {
-    void *p[9];
-    size_t b[9], off = 0;
+    void *p[8];
+    size_t b[8], off = 0;
     state_arrays(h, p, b);
     unsigned char *dst = (unsigned char *)h->ckpt[c];
-    const size_t real[9] = {4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n,
-                            4 * (size_t)h->ring_words, 4 * (size_t)h->sum_words, 8 * (size_t)h->n_nets,
+    const size_t real[8] = {4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n,
+                            4 * (size_t)h->ring_words, 8 * (size_t)h->n_nets,
                             4 * (size_t)h->n_nets, 8 * (size_t)h->n_nets};
-    for (int i = 0; i < 9; ++i) {
+    for (int i = 0; i < 8; ++i) {
         if (real[i]) SK(cudaMemcpyAsync(dst + off, p[i], real[i], cudaMemcpyDeviceToDevice, st));
         off += b[i];
     }
@@ -536,14 +686,14 @@ __global__ void k_sweep_set_step(int64_t *step, int *queue, int64_t v) {
 }
 
 int checkpoint_restore(eb_sweep *h, int c, int64_t step, cudaStream_t st) {
-    void *p[9];
-    size_t b[9], off = 0;
+    void *p[8];
+    size_t b[8], off = 0;
     state_arrays(h, p, b);
     const unsigned char *src = (const unsigned char *)h->ckpt[c];
-    const size_t real[9] = {4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n,
-                            4 * (size_t)h->ring_words, 4 * (size_t)h->sum_words, 8 * (size_t)h->n_nets,
+    const size_t real[8] = {4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n,
+                            4 * (size_t)h->ring_words, 8 * (size_t)h->n_nets,
                             4 * (size_t)h->n_nets, 8 * (size_t)h->n_nets};
-    for (int i = 0; i < 9; ++i) {
+    for (int i = 0; i < 8; ++i) {
         if (real[i]) SK(cudaMemcpyAsync(p[i], src + off, real[i], cudaMemcpyDeviceToDevice, st));
         off += b[i];
     }
@@ -729,7 +879,7 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
     std::vector<int32_t> grp_lo(n_steps_max + 2, 0);
     std::vector<int8_t> grp_n(n_steps_max + 2, 0);
     h->h_arr_step.assign(n_steps_max + 1, INT32_MAX);
-    int64_t dmax = 1;
+    int64_t dmax = 1, lag = INT32_MAX;
     {
         int64_t ka = 2;
         for (int64_t j = 1; j <= n_steps_max; ++j) {
@@ -741,15 +891,20 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
             if (grp_n[ka] == 0) grp_lo[ka] = (int32_t)j;
             if (++grp_n[ka] > kMaxGroups) { set_error("eb_sweep_build: dt too small for the delay grid"); return EB_ERR_UNSUPPORTED; }
             dmax = std::max(dmax, ka - j);
+            lag = std::min(lag, ka - j);
         }
     }
-    const int R = (int)dmax + 2;
+    // A window's sources precede it (at most `lag` steps, the fewest from a spike to its
+    // arrival); the ring holds the sources of its lists, then the spikes of the window
+    // being drained, while the next window's are written.
+    h->G.window = (int)std::max<int64_t>(1, std::min<int64_t>(kSweepWindow, lag));
+    const int R = (int)dmax + 1 + h->G.window;
     h->G.R = R;
     h->G.steps_max = (int)n_steps_max;
     h->G.dt_ms = h->dt * 1000.0f;
     h->G.integ = h->integ;
     // layout and input arrivals
-    int64_t src_off = 0, state_off = 0, in_off = 0, ring_off = 0, sum_off = 0, rec_off = 0;
+    int64_t src_off = 0, state_off = 0, in_off = 0, ring_off = 0, rec_off = 0;
     std::vector<int32_t> in_key;
     std::vector<uint16_t> in_src;
     h->max_n = 0;
@@ -761,8 +916,6 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
         state_off += S.n;
         S.ring_off = ring_off;
         ring_off += (int64_t)R * S.wn;
-        S.sum_off = sum_off;
-        sum_off += (int64_t)R * ((S.wn + 31) / 32);
         S.rec_off = rec_off;
         S.rec_cap = (int64_t)std::ceil((double)S.n * (double)n_steps_max * (double)h->dt * (double)max_rate_hz) + 64;
         rec_off += S.rec_cap;
@@ -798,7 +951,7 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
     }
     h->state_n = state_off;
     h->ring_words = ring_off;
-    h->sum_words = sum_off;
+    h->n_sources = src_off;
     h->h_in_key = in_key;
     h->G.n_total = state_off;
     int rc;
@@ -903,7 +1056,6 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
     if ((rc = h->upload((void **)&h->G.gI, nullptr, sizeof(float) * (size_t)state_off))) return rc;
     if ((rc = h->upload((void **)&h->G.refr, nullptr, sizeof(int32_t) * (size_t)state_off))) return rc;
     if ((rc = h->upload((void **)&h->G.ring, nullptr, sizeof(uint32_t) * (size_t)ring_off))) return rc;
-    if ((rc = h->upload((void **)&h->G.rsum, nullptr, sizeof(uint32_t) * (size_t)sum_off))) return rc;
     if ((rc = h->upload((void **)&h->G.grp_lo, grp_lo.data(), sizeof(int32_t) * grp_lo.size()))) return rc;
     if ((rc = h->upload((void **)&h->G.grp_n, grp_n.data(), sizeof(int8_t) * grp_n.size()))) return rc;
     if ((rc = h->upload((void **)&h->G.in_key, in_key.data(), sizeof(int32_t) * in_key.size()))) return rc;
@@ -937,7 +1089,6 @@ int eb_sweep_reset(eb_sweep *h) {
     SK(cudaMemsetAsync(h->G.gI, 0, sizeof(float) * ns, st));
     SK(cudaMemsetAsync(h->G.refr, 0xff, sizeof(int32_t) * ns, st));  // -1: never spiked
     SK(cudaMemsetAsync(h->G.ring, 0, sizeof(uint32_t) * (size_t)h->ring_words, st));
-    SK(cudaMemsetAsync(h->G.rsum, 0, sizeof(uint32_t) * (size_t)h->sum_words, st));
     SK(cudaMemsetAsync(h->G.in_cursor, 0, sizeof(int64_t) * h->n_nets, st));
     SK(cudaMemsetAsync(h->G.rec_cnt, 0, sizeof(uint32_t) * h->n_nets, st));
     SK(cudaMemsetAsync(h->G.rec_end, 0, sizeof(int32_t) * (size_t)h->n_nets * h->G.steps_max, st));
@@ -954,39 +1105,71 @@ int eb_sweep_reset(eb_sweep *h) {
 
 int eb_sweep_configure(eb_sweep *h, int block, int steps_per_launch) {
     if (!h || !h->built) { set_error("eb_sweep_configure: sweep not built"); return EB_ERR_STATE; }
+    SK(cudaSetDevice(h->device));
+    int nsm = 0;
+    SK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
+    // CTAs per network: with fewer networks than SMs, as many as leave each at least
+    // kTileMin neurons (below, a tile's update is shorter than what all CTAs repeat:
+    // @TILEMIN@), the SMs one CTA each, and a window of steps to meet in
+    int ctas = 1;
+    while (ctas < 8 && 2 * ctas * h->n_nets <= nsm && 2 * ctas * kTileMin <= h->max_n) ctas *= 2;
+    const int words = (h->max_n + 31) / 32;
+    int max_smem = 0;
+    SK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    auto tile_of = [&](int c) { return (words + c - 1) / c * 32; };
+    // sources a pass lists: 128, or 64 where the state needs the shared memory
+    auto smem_of = [&](int c, int cap) { return sweep_smem_bytes(tile_of(c), h->G.R, words, h->G.window, cap); };
+    const size_t room = (size_t)max_smem - 1024;
+    while (ctas < 8 && smem_of(ctas, 64) > room) ctas *= 2;
+    const int cap = smem_of(ctas, 128) <= room ? 128 : 64;
+    const int tile = tile_of(ctas);
     int nb = block ? block : h->block;
+    // threads per CTA unless the caller chose: two CTAs of 512 share an SM; a lone one
+    // takes 1,024 when its tile gives them two neurons each, and fewer than 512 only
+    // leave warps without a neuron out
+    if (!nb) {
+        nb = 512;
+        if ((int64_t)ctas * h->n_nets <= nsm && tile >= 2048) nb = 1024;
+        while (nb > 128 && nb / 2 >= tile) nb /= 2;
+    }
     if (nb != 128 && nb != 256 && nb != 512 && nb != 1024) { set_error("block must be 128, 256, 512 or 1024"); return EB_ERR_ARG; }
     if (steps_per_launch < 0) { set_error("steps_per_launch < 0"); return EB_ERR_ARG; }
-    const int npt = (h->max_n + nb - 1) / nb;  // neurons per thread
-    const int wc = npt * nb / 32;
-    const int swc = (wc + 31) / 32;
-    const size_t smem = 16 * (size_t)h->max_n + sizeof(uint32_t) * (size_t)h->G.R * (wc + swc) +
-                        sizeof(int32_t) * (3 * (size_t)kListCap + 1);
-    SweepFn f = sweep_fn(h->integ, false);
-    SK(cudaSetDevice(h->device));
-    if (smem > 48 * 1024) {
-        for (bool traj : {false, true}) {
-            cudaError_t e = cudaFuncSetAttribute((const void *)sweep_fn(h->integ, traj),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) {
-                set_error("sweep kernel: %zu bytes of shared memory unavailable (%s)", smem, cudaGetErrorString(e));
-                return EB_ERR_UNSUPPORTED;
-            }
+    const size_t smem = smem_of(ctas, cap);
+    // the largest any sweep of the process needs: another handle may have raised it
+    for (bool traj : {false, true}) {
+        const void *f = (const void *)sweep_fn(h->integ, traj, ctas > 1);
+        cudaFuncAttributes fa;
+        SK(cudaFuncGetAttributes(&fa, f));
+        if ((size_t)fa.maxDynamicSharedSizeBytes >= smem) continue;
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            set_error("sweep kernel: %zu bytes of shared memory unavailable (%s)", smem, cudaGetErrorString(e));
+            return EB_ERR_UNSUPPORTED;
         }
     }
-    int nsm = 0, occ = 0;
-    SK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
-    SK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, nb, smem));
+    int occ = 0;
+    SK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sweep_fn(h->integ, false, ctas > 1), nb, smem));
     if (occ < 1) {
         set_error("sweep kernel does not fit (block %d, %zu bytes of shared memory)", nb, smem);
         return EB_ERR_UNSUPPORTED;
     }
+    const int cl = ctas == 8 ? 3 : ctas / 2;  // log2
+    if (ctas > 1 && !h->tile_ptr[cl]) {
+        int rc = h->dalloc((void **)&h->tile_ptr[cl], sizeof(uint32_t) * (size_t)h->n_sources * (ctas + 1));
+        if (rc) return rc;
+        k_sweep_tiles<<<dim3(64, h->n_nets), 256, 0, h->stream>>>(h->G, ctas, h->tile_ptr[cl]);
+        SK(cudaGetLastError());
+    }
     h->block = nb;
-    h->npt = npt;
-    h->wc = wc;
-    h->swc = swc;
+    h->max_tile = tile;
+    h->wc = words;
     h->smem = smem;
-    h->grid = std::min(occ * nsm, h->n_nets);
+    h->G.ctas = ctas;
+    h->G.list_cap = cap;
+    h->G.tptr = ctas > 1 ? h->tile_ptr[cl] : h->G.optr;
+    h->G.tstride = ctas > 1 ? ctas + 1 : 1;
+    h->grid = ctas > 1 ? ctas * h->n_nets : std::min(occ * nsm, h->n_nets);
     if (steps_per_launch) h->steps_per_launch = steps_per_launch;
     if (h->graph) {
         cudaGraphExecDestroy(h->graph);

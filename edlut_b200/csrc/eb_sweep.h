@@ -15,7 +15,9 @@ namespace ebsw {
 using namespace eb;
 
 constexpr int kSweepMaxN = 16384;   // neurons per network
-constexpr int kListCap = 512;       // sources per delivery pass
+constexpr int kSweepWindow = 8;     // steps between meetings of a network's CTAs and record drains
+constexpr int kOwnObs = 1024;       // most observed neurons a network's threads record themselves
+constexpr int kTileMin = 512;       // fewest neurons a CTA of several per network is given
 constexpr int kBatch = 4;           // synapses per thread per delivery batch
 constexpr int kMaxGroups = 3;       // source steps arriving in one step
 constexpr int kMaxFrac = 4;         // steps with a partial refractory fraction
@@ -45,7 +47,6 @@ struct SweepNet {
     int64_t state_off;            // into V / refr / gE / gI
     int64_t in_off, n_in_spikes;  // into in_key / in_src
     int64_t ring_off;             // R * wn words
-    int64_t sum_off;              // R * ceil(wn / 32) words
     int64_t rec_off, rec_cap;     // into rec (uint16 neurons)
     float params[10];             // LIF .cfg order
     SweepLif L;
@@ -64,7 +65,7 @@ struct SweepDev {
     const float *w;
     float *V, *gE, *gI;
     int32_t *refr;
-    uint32_t *ring, *rsum;     // saved bitmask ring and summaries
+    uint32_t *ring;            // saved bitmask ring
     const int32_t *in_key;     // arrival step * 4 + phase, sorted per network
     const uint16_t *in_src;    // input neuron (local)
     int64_t *in_cursor;        // per network
@@ -77,6 +78,11 @@ struct SweepDev {
     int64_t *step;             // steps completed
     float dt_ms;
     int integ;
+    // launch shape: CTAs per network (a cluster when above 1), steps of a window, sources
+    // a delivery pass lists, and the first synapse of each source in each CTA's tile of
+    // targets: tptr[(source) * tstride + tile], relative to syn_off (optr for one CTA)
+    int ctas, window, list_cap, tstride;
+    const uint32_t *tptr;
     // observed membrane traces: trace[(net * steps_max + k - 1) * n_obs + m] = V of neuron obs[net * n_obs + m] after step k
     int n_obs;
     const int32_t *obs;
@@ -90,20 +96,23 @@ struct SweepDev {
 
 // Derivative of V (lif_deriv of the plain path) with the refractory test given as
 // a class: 0 none, 1 frozen (derivative 0), 2 scaled by f.
+template <int EN = -1>
 __device__ __forceinline__ float sw_deriv(const SweepLif &L, float V, float gE, float gI, int cls, float f) {
-    if (cls == 1) return 0.0f;
+    const int en = EN >= 0 ? EN : L.en;
     float current = 0.0f;
-    if (L.en & 1) current += gE * (L.e_exc - V);
-    if (L.en & 2) current += gI * (L.e_inh - V);
+    if (en & 1) current = gE * (L.e_exc - V);
+    if (en & 2) current += gI * (L.e_inh - V);
     const float full = (current + L.g_leak * (L.e_leak - V)) * L.inv_c_m;
-    return cls == 2 ? f * full : full;
+    return cls == 1 ? 0.0f : cls == 2 ? f * full : full;  // (f of class 0 is 1: the forward passes it as class 2)
 }
 
 // EvaluateTimeDependentEquation: g <- 0 below 1e-9, else g * factor.
+template <int EN = -1>
 __device__ __forceinline__ void sw_decay(const SweepLif &L, float &gE, float &gI) {
+    const int en = EN >= 0 ? EN : L.en;
     const float limit = 1e-9;
-    if (L.en & 1) { if (gE < limit) gE = 0.0f; else gE *= L.decay[0]; }
-    if (L.en & 2) { if (gI < limit) gI = 0.0f; else gI *= L.decay[1]; }
+    if (en & 1) { if (gE < limit) gE = 0.0f; else gE *= L.decay[0]; }
+    if (en & 2) { if (gI < limit) gI = 0.0f; else gI *= L.decay[1]; }
 }
 
 }  // namespace ebsw
@@ -132,9 +141,12 @@ struct eb_sweep {
     int64_t *perm = nullptr;            // sweep synapse position -> caller position
     int64_t steps_done = 0;
     bool needs_reset = false;
-    int64_t total_syn = 0, dev_bytes = 0, state_n = 0, ring_words = 0, sum_words = 0;
-    int max_n = 0;
-    int block = 512, npt = 0, wc = 0, swc = 0;
+    int64_t total_syn = 0, dev_bytes = 0, state_n = 0, ring_words = 0;
+    int64_t n_sources = 0;              // optr entries of all networks
+    int max_n = 0;                      // largest network
+    int block = 0;                      // threads per CTA (0 until chosen)
+    int max_tile = 0, wc = 0;           // neurons a CTA holds; ring words of a step
+    uint32_t *tile_ptr[4] = {};         // tptr of 2, 4 and 8 CTAs per network (built on first use)
     int steps_per_launch = 1000;
     int grid = 0;
     size_t smem = 0;

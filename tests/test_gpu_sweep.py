@@ -130,3 +130,45 @@ def test_errors_leave_the_sweep_usable():
     sw.run(nsteps)
     assert_network_matches(sw, 0, nsteps)
     sw.close()
+
+
+@pytest.mark.parametrize("n,observed", [(1023, 3), (1024, 1500), (2050, 200), (4100, 5), (8200, 2000)])
+def test_networks_split_over_a_cluster_match_solo_runs(n, observed):
+    # few networks of at least 2 x 512 neurons run on 2, 4 or 8 CTAs each (1,023 on one);
+    # the smaller network beside the large one leaves CTAs with few neurons or none.
+    # Observed neurons repeat, so that one thread owns several or the block reads them.
+    nsteps = 403
+    specs = sweep_networks(seed=n, n_networks=2, n_min=n, n_max=n + 1, t_end=nsteps * 1e-4)
+    specs[1] = sweep_networks(seed=n + 1, n_networks=1, n_min=n // 5, n_max=n // 5 + 1, t_end=nsteps * 1e-4)[0]
+    sw = make_sweep(specs, nsteps)
+    rng = np.random.default_rng(n)
+    obs = np.stack([rng.integers(0, s["n"], observed) for s in specs]).astype(np.int32)
+    sw.set_observed(obs)
+    sw.run(nsteps)
+    trace = sw.trace(nsteps)
+    spikes = 0
+    for i in range(len(specs)):
+        spikes += assert_network_matches(sw, i, nsteps)
+        from edlut_b200.simulation import Simulation
+        net, t, c = sw.solo_description(i)
+        sim = Simulation.from_description(net, record_capacity=4_000_000)
+        sim.inject_spikes(t, c)
+        sim.set_trace(0, specs[i]["n"], nsteps)
+        sim.run(nsteps)
+        np.testing.assert_array_equal(trace[i], sim.get_trace()[:, obs[i], 0])
+        sim.close()
+    assert spikes > 0
+    sw.close()
+
+
+def test_sweeps_of_different_sizes_live_side_by_side():
+    # a later, smaller sweep does not take the shared memory a larger one was given
+    nsteps = 200
+    big = make_sweep(sweep_networks(seed=3, n_networks=80, n_min=4000, n_max=4100, t_end=nsteps * 1e-4), nsteps)
+    small = make_sweep(sweep_networks(seed=4, n_networks=80, n_min=200, n_max=210, t_end=nsteps * 1e-4), nsteps)
+    small.run(nsteps)
+    big.run(nsteps)
+    assert_network_matches(big, 7, nsteps)
+    assert_network_matches(small, 7, nsteps)
+    big.close()
+    small.close()

@@ -17,7 +17,8 @@ void launch_flush_post(const PopDev &P, const NetDev &N, int max_chunks, uint32_
 // Weights of the synapses at target-major positions tpos[0..c) into / from w[0..c).
 void launch_weights_get(const SynRec *syn, const uint32_t *tpos, int64_t c, float *w, cudaStream_t st);
 void launch_weights_set(SynRec *syn, const uint32_t *tpos, int64_t c, const float *w, cudaStream_t st);
-void launch_advance(int64_t *step, int K, cudaStream_t st);
+// Advance the step counter by K (0: the kernels before did) and report to the host.
+void launch_advance(int64_t *step, int K, const NetDev &N, RunStatus *status, cudaStream_t st);
 
 constexpr int kMaxPersistPops = 16;
 // Host-built description of one network for the persistent kernel.

@@ -288,6 +288,8 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
     if ((rc = dalloc((void **)&d_step, sizeof(int64_t)))) return rc;
     CK(cudaMemsetAsync(d_step, 0, sizeof(int64_t), st));
     N.step = d_step;
+    CK(cudaHostAlloc((void **)&status, sizeof(RunStatus), cudaHostAllocPortable));
+    *status = RunStatus{0, 0};
     if ((rc = dalloc((void **)&N.cnt, sizeof(uint32_t) * (size_t)R * n_neurons))) return rc;
     CK(cudaMemsetAsync(N.cnt, 0, sizeof(uint32_t) * (size_t)R * n_neurons, st));
     if ((rc = dalloc((void **)&N.rec, sizeof(Arrival) * (size_t)R * std::max<int64_t>(cap_total, 1)))) return rc;
@@ -1000,7 +1002,7 @@ int eb_ctx::build_graph(int K) {
         }
     }
     const int kernels = enq_count + 1;
-    launch_advance(d_step, K, stream);
+    launch_advance(d_step, K, net, status, stream);
     CK(cudaStreamEndCapture(stream, &g));
     cudaGraphExec_t exec = nullptr;
     cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
@@ -1052,6 +1054,9 @@ int eb_ctx::run_async(int64_t n) {
             launches += 1;
             done += k;
         }
+        launch_advance(d_step, 0, net, status, stream);  // the kernel advanced the counter
+        CK(cudaGetLastError());
+        launches += 1;
         steps_done = k_end;
         return EB_OK;
     }
@@ -1072,7 +1077,7 @@ int eb_ctx::run_async(int64_t n) {
             }
             if (lazy_post) enqueue_flush(false);
         }
-        launch_advance(d_step, (int)n, stream);
+        launch_advance(d_step, (int)n, net, status, stream);
         CK(cudaStreamEndCapture(stream, &g));
         CK(cudaGraphInstantiate(&ge, g, 0));
         cudaGraphDestroy(g);
@@ -1105,7 +1110,7 @@ int eb_ctx::run_async(int64_t n) {
     while (done < n) {
         enq_count = 0;
         enqueue_step(0);
-        launch_advance(d_step, 1, stream);
+        launch_advance(d_step, 1, net, status, stream);
         if (lazy_post && ++steps_since_flush == kPostGraph) enqueue_flush(false);
         launches += enq_count + 1;
         done++;
@@ -1121,10 +1126,10 @@ int eb_ctx::sync() {
         int rc = prof_collect();
         if (rc) return rc;
     }
-    uint32_t f = 0;
-    CK(cudaMemcpy(&f, net.flags, sizeof(f), cudaMemcpyDeviceToHost));
+    const uint32_t f = status ? status->flags : 0u;
     if (f) {
         CK(cudaMemset(net.flags, 0, sizeof(uint32_t)));
+        status->flags = 0;
         if (f & FLAG_BDF_SINGULAR) { set_error("BDF Newton matrix not invertible"); return EB_ERR_NUMERIC; }
         if (f & FLAG_BUCKET_OVERFLOW) {
             set_error("arrival bucket overflow: a neuron received more spikes in one step than its bucket holds "
@@ -1207,6 +1212,7 @@ int eb_ctx::restore(int slot) {
     CK(cudaMemsetAsync(net.rec_count, 0, sizeof(unsigned long long), stream));
     rec_step_lo = steps_done;
     CK(cudaStreamSynchronize(stream));
+    status->rec_count = 0;
     return EB_OK;
 }
 
@@ -1221,6 +1227,7 @@ eb_ctx::~eb_ctx() {
     if (mon_file) std::fclose(mon_file);
     dfree_all();
     if (rec_host) cudaFreeHost(rec_host);
+    if (status) cudaFreeHost(status);
     if (own_stream && stream) cudaStreamDestroy(stream);
 }
 
@@ -1322,19 +1329,24 @@ int eb_inject_spikes(eb_ctx *ctx, int64_t n, const float *time_s, const int64_t 
             return EB_ERR_ARG;
         }
     }
+    const auto earlier = [](const PendingIn &a, const PendingIn &b) {
+        if (a.t != b.t) return a.t < b.t;
+        return a.seq < b.seq;
+    };
+    ctx->pending.reserve(ctx->pending.size() + (size_t)n);
+    bool sorted = true;  // lists come in time order as a rule
     for (int64_t i = 0; i < n; ++i) {
-        ctx->pending.push_back({time_s[i], cell[i], ctx->pending_seq++});
+        const PendingIn p{time_s[i], cell[i], ctx->pending_seq++};
+        sorted = sorted && (ctx->pending.empty() || !earlier(p, ctx->pending.back()));
+        ctx->pending.push_back(p);
         // a model neuron used as an input source can deliver twice in one step
         if (ctx->finalized && ctx->pops[ctx->pop_of[cell[i]]].kind != KIND_INPUT) {
-            for (auto &p : ctx->pops) p.dev.may_repeat = 1;
+            for (auto &q : ctx->pops) q.dev.may_repeat = 1;
             ctx->graphs_valid = false;
             ctx->pops_dirty = true;
         }
     }
-    std::stable_sort(ctx->pending.begin(), ctx->pending.end(), [](const PendingIn &a, const PendingIn &b) {
-        if (a.t != b.t) return a.t < b.t;
-        return a.seq < b.seq;
-    });
+    if (!sorted) std::stable_sort(ctx->pending.begin(), ctx->pending.end(), earlier);
     return EB_OK;
 }
 
@@ -1407,8 +1419,7 @@ int eb_get_spikes(eb_ctx *ctx, int64_t cap, int64_t *n, int64_t *step, int64_t *
     if (!ctx || !n) { set_error("bad argument"); return EB_ERR_ARG; }
     if (!ctx->finalized) { set_error("not finalized"); return EB_ERR_STATE; }
     CK(cudaStreamSynchronize(ctx->stream));
-    unsigned long long cnt = 0;
-    CK(cudaMemcpy(&cnt, ctx->net.rec_count, sizeof(cnt), cudaMemcpyDeviceToHost));
+    const unsigned long long cnt = ctx->status->rec_count;
     int64_t have = (int64_t)std::min<unsigned long long>(cnt, (unsigned long long)ctx->rec_cap);
     *n = have;
     if (have > cap) { set_error("eb_get_spikes: %lld spikes, buffer holds %lld", (long long)have, (long long)cap); return EB_ERR_OVERFLOW; }
@@ -1450,7 +1461,10 @@ int eb_get_spikes(eb_ctx *ctx, int64_t cap, int64_t *n, int64_t *step, int64_t *
     }
     ctx->spikes_drained += have;
     ctx->rec_step_lo = s_hi;
-    CK(cudaMemset(ctx->net.rec_count, 0, sizeof(unsigned long long)));
+    if (cnt) {
+        CK(cudaMemsetAsync(ctx->net.rec_count, 0, sizeof(unsigned long long), ctx->stream));
+        ctx->status->rec_count = 0;
+    }
     return EB_OK;
 }
 

@@ -72,6 +72,7 @@ struct eb_ctx {
     float *d_wstage = nullptr;    // weights on their way to or from the host (first use)
     eb::NetDev net{};
     int64_t *d_step = nullptr;
+    eb::RunStatus *status = nullptr;  // pinned, written by the device at the end of each run segment
     bool has_inputs = false;
     bool inputs_concurrent = false;  // input fan-out can overlap the neuron updates
     int input_threads = 32;

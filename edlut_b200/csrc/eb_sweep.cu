@@ -1305,21 +1305,41 @@ int eb_sweep_autotune(eb_sweep *h, int64_t trial_steps, int *best_block, int *be
 int eb_sweep_get_spikes(eb_sweep *h, int i, int64_t cap, int64_t *n, int32_t *step, int32_t *cell) {
     if (!h || !h->built || i < 0 || i >= h->n_nets || !n || cap < 0) { set_error("eb_sweep_get_spikes: bad argument"); return EB_ERR_ARG; }
     SK(cudaSetDevice(h->device));
-    SK(cudaStreamSynchronize(h->stream));
     const SweepNet &S = h->nets[i];
     const int64_t ns = h->steps_done;
-    std::vector<int32_t> end(ns);
-    if (ns) SK(cudaMemcpy(end.data(), h->G.rec_end + (int64_t)i * h->G.steps_max, sizeof(int32_t) * ns, cudaMemcpyDeviceToHost));
-    const int64_t cnt = ns ? (int64_t)(uint32_t)end[ns - 1] : 0;
+    // a size query reads the last step's count; a drain copies the steps' ends and as much
+    // of the record as the caller has room for at once, through pinned memory
+    int64_t room = std::min(cap, S.rec_cap);
+    if (room > kDrainAtOnce && ns) {  // far more room than spikes, maybe: ask first
+        int32_t c = 0;
+        SK(cudaMemcpyAsync(&c, h->G.rec_end + (int64_t)i * h->G.steps_max + ns - 1, sizeof(c), cudaMemcpyDeviceToHost, h->stream));
+        SK(cudaStreamSynchronize(h->stream));
+        room = std::min<int64_t>(room, std::max<int64_t>(1, (uint32_t)c));
+    }
+    const size_t end_bytes = (sizeof(int32_t) * (size_t)(room ? ns : 1) + 15) / 16 * 16;
+    const size_t need = end_bytes + sizeof(uint16_t) * (size_t)room;
+    if (need > h->pin_bytes) {
+        if (h->pin) cudaFreeHost(h->pin);
+        h->pin = nullptr;
+        h->pin_bytes = 0;
+        SK(cudaHostAlloc(&h->pin, need + need / 2, cudaHostAllocDefault));
+        h->pin_bytes = need + need / 2;
+    }
+    const int32_t *end = (const int32_t *)h->pin;
+    uint16_t *buf = (uint16_t *)((unsigned char *)h->pin + end_bytes);
+    const int32_t *row = h->G.rec_end + (int64_t)i * h->G.steps_max;
+    if (ns && room) SK(cudaMemcpyAsync(h->pin, row, sizeof(int32_t) * (size_t)ns, cudaMemcpyDeviceToHost, h->stream));
+    else if (ns) SK(cudaMemcpyAsync(h->pin, row + ns - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    if (ns && room) SK(cudaMemcpyAsync(buf, h->G.rec + S.rec_off, sizeof(uint16_t) * (size_t)room, cudaMemcpyDeviceToHost, h->stream));
+    SK(cudaStreamSynchronize(h->stream));
+    const int64_t cnt = ns ? (int64_t)(uint32_t)end[room ? ns - 1 : 0] : 0;
     *n = cnt;
     if (cnt > S.rec_cap) { set_error("network %d: spike record overflowed (raise max_rate_hz)", i); return EB_ERR_OVERFLOW; }
     if (cnt > cap) { set_error("eb_sweep_get_spikes: buffer holds %lld of %lld spikes", (long long)cap, (long long)cnt); return EB_ERR_OVERFLOW; }
-    std::vector<uint16_t> buf(cnt);
-    if (cnt) SK(cudaMemcpy(buf.data(), h->G.rec + S.rec_off, sizeof(uint16_t) * cnt, cudaMemcpyDeviceToHost));
+    if (!cnt) return EB_OK;
     int64_t b = 0;
     for (int64_t k = 0; k < ns; ++k) {
         const int64_t e = (uint32_t)end[k];
-        std::sort(buf.begin() + b, buf.begin() + e);  // within a step the record order is arbitrary
         for (int64_t q = b; q < e; ++q) {
             if (step) step[q] = (int32_t)(k + 1);
             if (cell) cell[q] = buf[q];

@@ -16,6 +16,7 @@ using namespace eb;
 
 constexpr int kSweepMaxN = 16384;   // neurons per network
 constexpr int kSweepWindow = 8;     // steps between meetings of a network's CTAs and record drains
+constexpr int64_t kDrainAtOnce = 1 << 20;  // spikes a drain copies without asking for their number first
 constexpr int kOwnObs = 1024;       // most observed neurons a network's threads record themselves
 constexpr int kTileMin = 512;       // fewest neurons a CTA of several per network is given
 constexpr int kBatch = 4;           // synapses per thread per delivery batch
@@ -166,9 +167,12 @@ struct eb_sweep {
     int32_t *obs_slot = nullptr;        // per neuron: observed slot or -1
     double *red_out = nullptr;          // [n_nets][4] parameter gradient sums
     int64_t traj_steps = 0;
+    void *pin = nullptr;                // spike read-back (pinned)
+    size_t pin_bytes = 0;
     ~eb_sweep() {
         if (graph) cudaGraphExecDestroy(graph);
         for (void *p : allocs) cudaFree(p);
+        if (pin) cudaFreeHost(pin);
         if (stream) cudaStreamDestroy(stream);
     }
     int dalloc(void **p, size_t b) {

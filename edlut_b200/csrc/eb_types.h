@@ -121,6 +121,13 @@ struct PopDev {
     int64_t mon_base;
 };
 
+// What the host reads after a run, in host memory that the device writes: the spike
+// records so far and the error flags.
+struct RunStatus {
+    unsigned long long rec_count;
+    uint32_t flags;
+};
+
 // Network-wide device pointers, passed by value to the kernels.
 struct NetDev {
     int64_t n_neurons;

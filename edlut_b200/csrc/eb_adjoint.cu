@@ -342,6 +342,25 @@ __global__ void k_adj_reduce(const SweepNet *nets, int64_t Nt, const double *gac
     }
 }
 
+__global__ void __launch_bounds__(256) k_adj_obs(SweepDev G, const SweepNet *nets, int32_t *obs_slot) {
+    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= (int64_t)G.n_nets * G.n_obs) return;
+    const int net = (int)(x / G.n_obs), m = (int)(x % G.n_obs);
+    atomicMax(obs_slot + nets[net].state_off + G.obs[x], m);
+}
+
+// Adjoints and gradient sums to zero in one launch.
+__global__ void __launch_bounds__(256) k_adj_clear(int64_t Nt, float *lamV, float *lamE, float *lamI, double *gacc, int64_t m,
+                                                   float *gw, uint32_t *flags) {
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < Nt; i += stride) {
+        lamV[i] = lamE[i] = lamI[i] = 0.0f;
+        gacc[i] = gacc[Nt + i] = gacc[2 * Nt + i] = gacc[3 * Nt + i] = 0.0;
+    }
+    for (int64_t i = i0; i < m; i += stride) gw[i] = 0.0f;
+    if (i0 == 0) *flags = 0u;
+}
+
 __global__ void k_perm_scatter_grad(const int64_t *perm, int64_t m, const float *src, float *dst) {
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < m; p += (int64_t)gridDim.x * blockDim.x)
         dst[perm[p]] = src[p];
@@ -395,14 +414,13 @@ extern "C" int eb_sweep_adjoint(eb_sweep *h, const float *grad_trace, int gt_on_
         if ((rc = adj_alloc(h, (void **)&h->obs_slot, sizeof(int32_t) * (size_t)Nt))) return rc;
         if ((rc = adj_alloc(h, (void **)&h->red_out, sizeof(double) * 4 * (size_t)h->n_nets))) return rc;
     }
-    // observed slot of every neuron (-1: not observed)
-    {
-        std::vector<int32_t> slot(Nt, -1);
+    if ((rc = upload_params(h, st))) return rc;
+    if (!h->obs_slot_ok) {  // observed slot of every neuron (-1: not observed), the last one of several
         const int m = h->G.n_obs;
-        for (int i = 0; i < h->n_nets; ++i)
-            for (int q = 0; q < m; ++q) slot[h->nets[i].state_off + h->h_obs[(size_t)i * m + q]] = q;
-        SK(cudaMemcpyAsync(h->obs_slot, slot.data(), sizeof(int32_t) * Nt, cudaMemcpyHostToDevice, st));
-        SK(cudaStreamSynchronize(st));
+        SK(cudaMemsetAsync(h->obs_slot, 0xff, sizeof(int32_t) * (size_t)Nt, st));
+        k_adj_obs<<<(unsigned)(((int64_t)h->n_nets * m + 255) / 256), 256, 0, st>>>(h->G, h->d_nets, h->obs_slot);
+        SK(cudaGetLastError());
+        h->obs_slot_ok = true;
     }
     const float *gt = grad_trace;
     float *gt_tmp = nullptr;
@@ -412,12 +430,8 @@ extern "C" int eb_sweep_adjoint(eb_sweep *h, const float *grad_trace, int gt_on_
         SK(cudaMemcpyAsync(gt_tmp, grad_trace, sizeof(float) * gt_n, cudaMemcpyHostToDevice, st));
         gt = gt_tmp;
     }
-    SK(cudaMemsetAsync(h->lamV, 0, sizeof(float) * Nt, st));
-    SK(cudaMemsetAsync(h->lamE, 0, sizeof(float) * Nt, st));
-    SK(cudaMemsetAsync(h->lamI, 0, sizeof(float) * Nt, st));
-    SK(cudaMemsetAsync(h->gacc, 0, sizeof(double) * 4 * Nt, st));
-    SK(cudaMemsetAsync(h->gw_sorted, 0, sizeof(float) * (size_t)std::max<int64_t>(1, h->total_syn), st));
-    SK(cudaMemsetAsync(h->G.flags, 0, sizeof(uint32_t), st));
+    k_adj_clear<<<148 * 4, 256, 0, st>>>(Nt, h->lamV, h->lamE, h->lamI, h->gacc, h->total_syn, h->gw_sorted, h->G.flags);
+    SK(cudaGetLastError());
     const AdjFn fa = adj_fn(h->integ);
     const dim3 ga((h->max_n + 255) / 256, h->n_nets);
     const int parts = std::max(1, (2 * 148 + h->n_nets - 1) / h->n_nets);

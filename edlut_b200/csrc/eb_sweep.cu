@@ -599,6 +599,32 @@ __global__ void __launch_bounds__(1024) k_sweep(SweepDev G, int nsteps, int max_
     }
 }
 
+// The initial state of every network (blockIdx.y): V = E_leak, no conductance, never
+// spiked, empty ring and records, step 0.  (Record ends are written before they are read.)
+__global__ void __launch_bounds__(256) k_sweep_reset(SweepDev G) {
+    const int net = blockIdx.y;
+    const SweepNet &S = G.nets[net];
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (int i = i0; i < S.n; i += stride) {
+        const int64_t o = S.state_off + i;
+        G.V[o] = S.L.e_leak;
+        G.gE[o] = 0.0f;
+        G.gI[o] = 0.0f;
+        G.refr[o] = -1;
+    }
+    for (int64_t x = i0; x < (int64_t)G.R * S.wn; x += stride) G.ring[S.ring_off + x] = 0u;
+    if (i0 == 0) {
+        G.in_cursor[net] = 0;
+        G.rec_cnt[net] = 0u;
+        G.events[net] = 0ull;
+        if (net == 0) {
+            *G.flags = 0u;
+            *G.queue = 0;
+            *G.step = 0;
+        }
+    }
+}
+
 // After a chunk: advance the step counter and re-arm the network queue.
 __global__ void k_sweep_advance(int64_t *step, int *queue, int nsteps) {
     *step += nsteps;
@@ -630,6 +656,12 @@ SweepFn sweep_fn(int integ, bool traj, bool clustered) {
 
 namespace ebsw {
 
+// (pointers and sizes of the arrays that k_sweep_copy moves)
+struct StateCopy {
+    uint32_t *live[8], *saved[8];
+    int64_t words[8];
+};
+
 int enqueue_chunk(eb_sweep *h, int nsteps, cudaStream_t st, bool traj, int64_t traj_k0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(h->grid);
@@ -648,57 +680,62 @@ int enqueue_chunk(eb_sweep *h, int nsteps, cudaStream_t st, bool traj, int64_t t
     return EB_OK;
 }
 
-// The arrays that make up the dynamic state, in checkpoint order.
-static void state_arrays(eb_sweep *h, void **ptr, size_t *bytes) {
+// The arrays that make up the dynamic state, in checkpoint order, and their places in a
+// checkpoint slot (256-byte aligned).  All are whole 32-bit words.
+constexpr int kStateArrays = 8;
+
+static size_t state_arrays(eb_sweep *h, StateCopy &c, void *slot) {
     const size_t nt = (size_t)h->state_n, B = (size_t)h->n_nets;
-    void *p[8] = {h->G.V, h->G.gE, h->G.gI, h->G.refr, h->G.ring, h->G.in_cursor, h->G.rec_cnt, h->G.events};
-    size_t b[8] = {4 * nt, 4 * nt, 4 * nt, 4 * nt, 4 * (size_t)h->ring_words, 8 * B, 4 * B, 8 * B};
-    for (int i = 0; i < 8; ++i) { ptr[i] = p[i]; bytes[i] = (b[i] + 255) / 256 * 256; }
-    for (int i = 0; i < 8; ++i) bytes[i] = b[i] ? bytes[i] : 0;
+    void *p[kStateArrays] = {h->G.V, h->G.gE, h->G.gI, h->G.refr, h->G.ring, h->G.in_cursor, h->G.rec_cnt, h->G.events};
+    const size_t words[kStateArrays] = {nt, nt, nt, nt, (size_t)h->ring_words, 2 * B, B, 2 * B};
+    size_t off = 0;
+    for (int i = 0; i < kStateArrays; ++i) {
+        c.live[i] = (uint32_t *)p[i];
+        c.saved[i] = (uint32_t *)slot + off;
+        c.words[i] = (int64_t)words[i];
+        off += (words[i] + 63) / 64 * 64;
+    }
+    return 4 * off;
 }
 
 size_t checkpoint_bytes(eb_sweep *h) {
-    void *p[8];
-    size_t b[8], t = 0;
-    state_arrays(h, p, b);
-    for (size_t x : b) t += x;
-    return t;
+    StateCopy c;
+    return state_arrays(h, c, nullptr);
 }
 
-int checkpoint_save(eb_sweep *h, int c, cudaStream_t st) {
-    void *p[8];
-    size_t b[8], off = 0;
-    state_arrays(h, p, b);
-    unsigned char *dst = (unsigned char *)h->ckpt[c];
-    const size_t real[8] = {4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n,
-                            4 * (size_t)h->ring_words, 8 * (size_t)h->n_nets,
-                            4 * (size_t)h->n_nets, 8 * (size_t)h->n_nets};
-    for (int i = 0; i < 8; ++i) {
-        if (real[i]) SK(cudaMemcpyAsync(dst + off, p[i], real[i], cudaMemcpyDeviceToDevice, st));
-        off += b[i];
+// All arrays of the state in one launch (eight copies cost the host 3 us each, and a
+// segment of the adjoint has two such sets); step >= 0 also sets the step counter and
+// re-arms the network queue.
+__global__ void __launch_bounds__(256) k_sweep_copy(StateCopy c, int restore, int64_t step, int64_t *d_step, int *queue) {
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int a = 0; a < kStateArrays; ++a) {
+        uint32_t *dst = restore ? c.live[a] : c.saved[a];
+        const uint32_t *src = restore ? c.saved[a] : c.live[a];
+        for (int64_t i = i0; i < c.words[a]; i += stride) dst[i] = src[i];
     }
+    if (i0 == 0 && step >= 0) {
+        *d_step = step;
+        *queue = 0;
+    }
+}
+
+static int checkpoint_copy(eb_sweep *h, int slot, int restore, int64_t step, cudaStream_t st) {
+    StateCopy c;
+    const size_t bytes = state_arrays(h, c, h->ckpt[slot]);
+    const int blocks = (int)std::min<size_t>(148 * 4, bytes / 4096 + 1);
+    k_sweep_copy<<<blocks, 256, 0, st>>>(c, restore, step, h->G.step, h->G.queue);
+    SK(cudaGetLastError());
     return EB_OK;
 }
 
-__global__ void k_sweep_set_step(int64_t *step, int *queue, int64_t v) {
-    *step = v;
-    *queue = 0;
-}
+int checkpoint_save(eb_sweep *h, int c, cudaStream_t st) { return checkpoint_copy(h, c, 0, -1, st); }
 
-int checkpoint_restore(eb_sweep *h, int c, int64_t step, cudaStream_t st) {
-    void *p[8];
-    size_t b[8], off = 0;
-    state_arrays(h, p, b);
-    const unsigned char *src = (const unsigned char *)h->ckpt[c];
-    const size_t real[8] = {4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n, 4 * (size_t)h->state_n,
-                            4 * (size_t)h->ring_words, 8 * (size_t)h->n_nets,
-                            4 * (size_t)h->n_nets, 8 * (size_t)h->n_nets};
-    for (int i = 0; i < 8; ++i) {
-        if (real[i]) SK(cudaMemcpyAsync(p[i], src + off, real[i], cudaMemcpyDeviceToDevice, st));
-        off += b[i];
-    }
-    k_sweep_set_step<<<1, 1, 0, st>>>(h->G.step, h->G.queue, step);
-    SK(cudaGetLastError());
+int checkpoint_restore(eb_sweep *h, int c, int64_t step, cudaStream_t st) { return checkpoint_copy(h, c, 1, step, st); }
+
+int upload_params(eb_sweep *h, cudaStream_t st) {
+    if (!h->nets_dirty) return EB_OK;
+    SK(cudaMemcpyAsync(h->d_nets, h->nets.data(), sizeof(SweepNet) * h->nets.size(), cudaMemcpyHostToDevice, st));
+    h->nets_dirty = false;
     return EB_OK;
 }
 
@@ -1048,9 +1085,6 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
         if ((rc = h->upload((void **)&h->perm, perm.data(), sizeof(int64_t) * perm.size()))) return rc;
     }
     // state and tables
-    h->v_init.assign(state_off, 0.0f);
-    for (int i = 0; i < N; ++i)
-        for (int j = 0; j < h->nets[i].n; ++j) h->v_init[h->nets[i].state_off + j] = h->nets[i].L.e_leak;
     if ((rc = h->upload((void **)&h->G.V, nullptr, sizeof(float) * (size_t)state_off))) return rc;
     if ((rc = h->upload((void **)&h->G.gE, nullptr, sizeof(float) * (size_t)state_off))) return rc;
     if ((rc = h->upload((void **)&h->G.gI, nullptr, sizeof(float) * (size_t)state_off))) return rc;
@@ -1082,21 +1116,11 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
 int eb_sweep_reset(eb_sweep *h) {
     if (!h || !h->built) { set_error("eb_sweep_reset: sweep not built"); return EB_ERR_STATE; }
     SK(cudaSetDevice(h->device));
-    cudaStream_t st = h->stream;
-    const size_t ns = (size_t)h->state_n;
-    SK(cudaMemcpyAsync(h->G.V, h->v_init.data(), sizeof(float) * ns, cudaMemcpyHostToDevice, st));
-    SK(cudaMemsetAsync(h->G.gE, 0, sizeof(float) * ns, st));
-    SK(cudaMemsetAsync(h->G.gI, 0, sizeof(float) * ns, st));
-    SK(cudaMemsetAsync(h->G.refr, 0xff, sizeof(int32_t) * ns, st));  // -1: never spiked
-    SK(cudaMemsetAsync(h->G.ring, 0, sizeof(uint32_t) * (size_t)h->ring_words, st));
-    SK(cudaMemsetAsync(h->G.in_cursor, 0, sizeof(int64_t) * h->n_nets, st));
-    SK(cudaMemsetAsync(h->G.rec_cnt, 0, sizeof(uint32_t) * h->n_nets, st));
-    SK(cudaMemsetAsync(h->G.rec_end, 0, sizeof(int32_t) * (size_t)h->n_nets * h->G.steps_max, st));
-    SK(cudaMemsetAsync(h->G.events, 0, sizeof(unsigned long long) * h->n_nets, st));
-    SK(cudaMemsetAsync(h->G.flags, 0, sizeof(uint32_t), st));
-    SK(cudaMemsetAsync(h->G.queue, 0, sizeof(int), st));
-    SK(cudaMemsetAsync(h->G.step, 0, sizeof(int64_t), st));
-    SK(cudaStreamSynchronize(st));
+    int rc = upload_params(h, h->stream);
+    if (rc) return rc;
+    k_sweep_reset<<<dim3(8, h->n_nets), 256, 0, h->stream>>>(h->G);
+    SK(cudaGetLastError());
+    SK(cudaStreamSynchronize(h->stream));
     h->steps_done = 0;
     h->needs_reset = false;
     h->ckpt_upto = h->ckpt_every > 0 ? 0 : -1;
@@ -1109,8 +1133,11 @@ int eb_sweep_configure(eb_sweep *h, int block, int steps_per_launch) {
     int nsm = 0;
     SK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
     // CTAs per network: with fewer networks than SMs, as many as leave each at least
-    // kTileMin neurons (below, a tile's update is shorter than what all CTAs repeat:
-    // @TILEMIN@), the SMs one CTA each, and a window of steps to meet in
+    // kTileMin neurons on average of the largest network, and the SMs one CTA each.  Each
+    // halving of the tile halves the update, while listing and meeting repeat: 24
+    // networks of up to 1,500, RK4, 500 steps with read-backs: 1.97 ms on one CTA, 1.77
+    // on two, 1.58 on four; 8 networks of up to 10,000, a fitting step: 14.4 ms on two,
+    // 9.2 on eight.
     int ctas = 1;
     while (ctas < 8 && 2 * ctas * h->n_nets <= nsm && 2 * ctas * kTileMin <= h->max_n) ctas *= 2;
     const int words = (h->max_n + 31) / 32;
@@ -1187,6 +1214,7 @@ int eb_sweep_run_async(eb_sweep *h, int64_t n_steps) {
         return EB_ERR_ARG;
     }
     SK(cudaSetDevice(h->device));
+    if (int rc = upload_params(h, h->stream)) return rc;
     if (h->ckpt_every > 0) {
         // chunks aligned to the checkpoint interval, the state saved before each
         const int E = h->ckpt_every;
@@ -1427,12 +1455,7 @@ int eb_sweep_set_params(eb_sweep *h, int i, const float *lif_params) {
     if (rc) return rc;
     S.L = L;
     for (int j = 0; j < 10; ++j) S.params[j] = lif_params[j];
-    if (h->built) {
-        SK(cudaSetDevice(h->device));
-        SK(cudaStreamSynchronize(h->stream));
-        SK(cudaMemcpy(h->d_nets + i, &S, sizeof(SweepNet), cudaMemcpyHostToDevice));
-        for (int j = 0; j < S.n; ++j) h->v_init[S.state_off + j] = L.e_leak;
-    }
+    h->nets_dirty = h->built;  // all changed networks go to the device at once, before the next launch
     return EB_OK;
 }
 
@@ -1496,6 +1519,7 @@ int eb_sweep_set_observed(eb_sweep *h, int m, const int32_t *idx) {
         h->G.trace = d_trace;
     }
     h->G.n_obs = m;
+    h->obs_slot_ok = false;
     h->h_obs.assign(idx, idx + (size_t)h->n_nets * m);
     if (h->graph) {
         cudaGraphExecDestroy(h->graph);

@@ -18,7 +18,7 @@ constexpr int kSweepMaxN = 16384;   // neurons per network
 constexpr int kSweepWindow = 8;     // steps between meetings of a network's CTAs and record drains
 constexpr int64_t kDrainAtOnce = 1 << 20;  // spikes a drain copies without asking for their number first
 constexpr int kOwnObs = 1024;       // most observed neurons a network's threads record themselves
-constexpr int kTileMin = 512;       // fewest neurons a CTA of several per network is given
+constexpr int kTileMin = 256;       // fewest neurons a CTA of several per network is given
 constexpr int kBatch = 4;           // synapses per thread per delivery batch
 constexpr int kMaxGroups = 3;       // source steps arriving in one step
 constexpr int kMaxFrac = 4;         // steps with a partial refractory fraction
@@ -135,7 +135,7 @@ struct eb_sweep {
     ebsw::SweepDev G{};
     ebsw::SweepNet *d_nets = nullptr;
     std::vector<void *> allocs;
-    std::vector<float> v_init;
+    bool nets_dirty = false;            // parameters changed since the device's copy
     std::vector<int32_t> h_in_key;      // host copy of the input arrival keys
     std::vector<int32_t> h_arr_step;    // arrival step of the spikes of each source step
     int32_t *d_arr_step = nullptr;
@@ -165,6 +165,7 @@ struct eb_sweep {
     float *muE = nullptr, *muI = nullptr;
     float *gw_sorted = nullptr;
     int32_t *obs_slot = nullptr;        // per neuron: observed slot or -1
+    bool obs_slot_ok = false;           // obs_slot is that of the observed neurons set last
     double *red_out = nullptr;          // [n_nets][4] parameter gradient sums
     int64_t traj_steps = 0;
     void *pin = nullptr;                // spike read-back (pinned)
@@ -210,4 +211,6 @@ int enqueue_chunk(eb_sweep *h, int nsteps, cudaStream_t st, bool traj = false, i
 size_t checkpoint_bytes(eb_sweep *h);
 int checkpoint_save(eb_sweep *h, int c, cudaStream_t st);
 int checkpoint_restore(eb_sweep *h, int c, int64_t step, cudaStream_t st);
+// Parameters set since the last launch, to the device.
+int upload_params(eb_sweep *h, cudaStream_t st);
 }  // namespace ebsw

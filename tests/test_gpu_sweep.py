@@ -132,9 +132,9 @@ def test_errors_leave_the_sweep_usable():
     sw.close()
 
 
-@pytest.mark.parametrize("n,observed", [(1023, 3), (1024, 1500), (2050, 200), (4100, 5), (8200, 2000)])
+@pytest.mark.parametrize("n,observed", [(511, 3), (512, 1500), (1030, 200), (2050, 5), (8200, 2000)])
 def test_networks_split_over_a_cluster_match_solo_runs(n, observed):
-    # few networks of at least 2 x 512 neurons run on 2, 4 or 8 CTAs each (1,023 on one);
+    # few networks of at least 2 x 256 neurons run on 2, 4 or 8 CTAs each (511 on one);
     # the smaller network beside the large one leaves CTAs with few neurons or none.
     # Observed neurons repeat, so that one thread owns several or the block reads them.
     nsteps = 403

@@ -22,12 +22,10 @@ constexpr float kHHMinV = -90.0f;
 
 // ExponentialTable::GetResult (include/simulation/ExponentialTable.h:92-103).
 __device__ __forceinline__ float expt(const PopDev &P, float v) {
-    if (v >= kExptMin && v <= kExptMax) {
-        int pos = (int)((v - kExptMin) * P.expt_aux);
-        return __ldg(P.exp_table + pos);
-    }
+    const bool in = v >= kExptMin && v <= kExptMax;
+    const float t = __ldg(P.exp_table + (in ? (int)((v - kExptMin) * P.expt_aux) : 0));
     if (v > kExptMax) return (float)exp((double)v);
-    return 0.0f;
+    return in ? t : 0.0f;
 }
 
 __device__ __forceinline__ float nmda_inf(const PopDev &P, float v, float e_inh) {
@@ -88,29 +86,22 @@ __device__ __forceinline__ void lif_deriv(const PopDev &P, const float *x, float
 template <int EN = -1>
 __device__ __forceinline__ void adex_deriv(const PopDev &P, const float *x, float *dx) {
     const float *p = P.p;
-    const float a = p[0], slope = p[2], vthr = p[3], eexc = p[5], einh = p[6], eleak = p[8], gl = p[9];
+    const float a = p[0], vthr = p[3], eexc = p[5], einh = p[6], eleak = p[8], gl = p[9];
     const int en = en_mask<EN>(P);
-    // P.adex_vmax = vthr + 6 * slope and P.adex_glslope = gl * slope: the same float
-    // operations, evaluated once on the host
-    if (x[0] <= P.adex_vmax) {
-        float current = 0.0f;
-        if (en & 1) current += x[2] * (eexc - x[0]);
-        if (en & 2) current += x[3] * (einh - x[0]);
-        if (en & 4) current += x[4] * nmda_inf(P, x[0], einh) * (eexc - x[0]);
-        dx[0] = (gl * (eleak - x[0]) + P.adex_glslope * expt(P, (x[0] - vthr) * P.inv_slope) - x[1] + current) * P.inv_c_m;
-        dx[1] = (a * (x[0] - eleak) - x[1]) * P.inv_tau_w;
-    } else if (x[0] <= 0.0f) {
-        const float Vm = vthr + 6 * slope;
-        float current = 0.0f;
-        if (en & 1) current += x[2] * (eexc - Vm);
-        if (en & 2) current += x[3] * (einh - Vm);
-        if (en & 4) current += x[4] * nmda_inf(P, Vm, einh) * (eexc - Vm);
-        dx[0] = (gl * (eleak - Vm) + gl * slope * expt(P, (Vm - vthr) * P.inv_slope) - x[1] + current) * P.inv_c_m;
-        dx[1] = (a * (x[0] - eleak) - x[1]) * P.inv_tau_w;
-    } else {
-        dx[0] = 0.0f;
-        dx[1] = 0.0f;
-    }
+    // The reference's three cases (V up to vthr + 6 slope, above it up to 0, above 0) by
+    // selection: the second is the first with V held at vthr + 6 slope in dV/dt, the third
+    // all zero.  P.adex_vmax = vthr + 6 * slope and P.adex_glslope = gl * slope are the
+    // same float operations, evaluated once on the host.
+    const bool low = x[0] <= P.adex_vmax, alive = low || x[0] <= 0.0f;
+    const float V = low ? x[0] : P.adex_vmax;
+    float current = 0.0f;
+    if (en & 1) current += x[2] * (eexc - V);
+    if (en & 2) current += x[3] * (einh - V);
+    if (en & 4) current += x[4] * nmda_inf(P, V, einh) * (eexc - V);
+    const float dV = (gl * (eleak - V) + P.adex_glslope * expt(P, (V - vthr) * P.inv_slope) - x[1] + current) * P.inv_c_m;
+    const float dw = (a * (x[0] - eleak) - x[1]) * P.inv_tau_w;
+    dx[0] = alive ? dV : 0.0f;
+    dx[1] = alive ? dw : 0.0f;
 }
 
 // --------------------------------------------------------------------- HH --

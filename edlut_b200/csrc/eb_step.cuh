@@ -570,8 +570,8 @@ __device__ __forceinline__ void update_narrow_tile(const PopDev &P, const NetDev
 //   Bound by the latency of the warp's chain: 1,000 LIF neurons, 3,000 steps 4.37 ->
 // 3.32 ms; 2,501 AdEx neurons with STDP, 500 steps 3.62 -> 2.42 ms; HH, 3,001 neurons
 // 12.9 -> 11.8 us a step, 100,000 29.7 -> 28.2.  Large LIF and AdEx populations are
-// bound by issue at 40 registers, where the staging spills 250 bytes: they keep the
-// per-step fold (250,000 granule cells 5.98 us a step, 6.16 staged).
+// bound by issue, and the staging spills 250 bytes at their registers: they keep the
+// per-step fold (250,000 granule cells at 40 registers: 5.98 us a step, 6.16 staged).
 template <int CAP>
 struct NarrowStage {
     Arrival arr[CAP];
@@ -744,12 +744,13 @@ __device__ __forceinline__ void narrow_window(const PopDev &P, const NetDev &N, 
 // HH under BDF holds the Newton state (Jacobian, inverse, history) in about 120
 // registers, which leaves 2 blocks per SM; bounded to 3 blocks (80 registers, a
 // 44-byte spill) a 100k-neuron population fits one wave and its steps take a
-// quarter less time.  LIF and AdEx under the explicit methods are bounded to 6
-// blocks (40 registers, spills of 8-12 bytes): a fifth more resident neurons than
-// at the compiler's 48, so a 250k-neuron population takes 1.06 waves, not 1.32.
+// quarter less time.  LIF and AdEx under the explicit methods are bounded to 5
+// blocks of 256 (48 registers): they are bound by issue, and at 40 registers a fifth
+// of the instructions re-read parameters (250,000 granule cells beside 40 Purkinje
+// cells: 5.96 us a step at 40 registers, 5.38 at 48, 5.46 at 54).
 // EN >= 0: the population's enabled conductance types fixed at compile time.
 constexpr int narrow_min_blocks(int kind, int integ) {
-    return (kind == KIND_HH && integ == INTEG_BDF) ? 3 : (kind != KIND_HH && integ != INTEG_BDF) ? 6 : 0;
+    return (kind == KIND_HH && integ == INTEG_BDF) ? 3 : (kind != KIND_HH && integ != INTEG_BDF) ? 5 : 0;
 }
 
 template <int KIND, int INTEG, int EN, int MON, bool SMALL>

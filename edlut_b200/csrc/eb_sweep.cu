@@ -19,9 +19,9 @@
 //      memory.  A spike is needed `lag` steps later, so the steps of a window of up to
 //      8 are listed at its start, a warp each, and the listed rows prefetched into L2.
 //      Every thread loads a batch of the listed sources' synapses (target, weight) at
-//      once, then the batch is applied one source at a time with a barrier in between:
-//      targets of one source are distinct, so each target receives its additions in
-//      list order without atomics (src/spike/PropagatedSpikeGroup.cpp:112-149);
+//      once, then the batch is applied one source at a time, or in rounds of bids when
+//      there are many (deliver_batch), so that each target receives its additions in
+//      list order without float atomics (src/spike/PropagatedSpikeGroup.cpp:112-149);
 //   2. update: each thread advances neurons tid, tid + blockDim, ... of its tile (the
 //      state -- V, refractory counter, gE, gI -- lives in shared memory for the chunk)
 //      with the model/integrator arithmetic of the plain path, with the refractory
@@ -194,6 +194,7 @@ struct SweepList {
 struct SweepSmem {
     float4 *x;              // [tile] V, gE, gI, refractory counter (integer bits)
     uint32_t *ring;         // [R][wc] spike bitmasks of the whole network
+    uint32_t *bid;          // [kBidSlots] lowest source rank bidding for a target (kNoBid between batches)
     int32_t *lists;         // the lists of a window's steps
     int cap;
     __device__ SweepList list(int s) const {
@@ -203,7 +204,7 @@ struct SweepSmem {
 };
 
 size_t sweep_smem_bytes(int tile, int R, int wc, int window, int cap) {
-    return 16 * (size_t)tile + sizeof(uint32_t) * (size_t)R * wc + window * sizeof(int32_t) * (3 * (size_t)cap + 1);
+    return 16 * (size_t)tile + sizeof(uint32_t) * ((size_t)R * wc + kBidSlots) + window * sizeof(int32_t) * (3 * (size_t)cap + 1);
 }
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -313,6 +314,77 @@ __device__ __forceinline__ int list_step(const SweepDev &G, const SweepSmem &M, 
     }
     if (lane == 0 && cnt > 0) B.off[cnt] = carry;
     return pos;
+}
+
+// Deliver entries e0 .. of the listed sources' flattened synapses, NB a thread, by the
+// whole block.  A target receives its additions in list order without atomics on
+// floats: a few sources go one at a time with a barrier in between (one source's
+// targets are distinct).  Many sources -- the bursts of a large network, whose rows in
+// a tile are short -- go in rounds instead: every pending entry bids its source's rank
+// for its target's slot, the lowest rank of a slot is added, the others bid again.  A
+// batch takes as many rounds as its most frequent target has entries, not one per
+// source (slots shared by several targets only make an entry wait).  A fitting step of
+// 8 networks of up to 10,000 neurons: 9.2 -> 7.4 ms; 600 networks: 6.5 -> 6.3 ms.
+template <int NB>
+__device__ __forceinline__ void deliver_batch(const SweepSmem &M, const SweepList &B, int sources, int e0, int total,
+                                              const uint16_t *tg, const float *ww, int n_exc, int n, int first) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    int t[NB], rk[NB];
+    float w[NB];
+    bool inh[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int e = e0 + q * nt + tid;
+        rk[q] = -1;
+        t[q] = 0;
+        w[q] = 0.0f;
+        inh[q] = false;
+        if (e < total) {
+            const int a = list_rank(B.off, sources, e);
+            const uint32_t o = B.base[a] + (uint32_t)(e - B.off[a]);
+            t[q] = (int)__ldg(tg + o) - first;
+            w[q] = __ldg(ww + o);
+            const int x = B.src[a];
+            inh[q] = x >= n_exc && x < n;
+            rk[q] = a;
+        }
+    }
+    auto add = [&](int q) {
+        float4 &x = M.x[t[q]];
+        if (inh[q]) x.z += w[q];
+        else x.y += w[q];
+    };
+    const int r_lo = list_rank(B.off, sources, e0);
+    const int r_hi = list_rank(B.off, sources, min(e0 + NB * nt, total) - 1);
+    if (r_hi - r_lo < kRoundSources) {
+        for (int a = r_lo; a <= r_hi; ++a) {
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+                if (rk[q] == a) add(q);
+            __syncthreads();
+        }
+        return;
+    }
+    bool pending = true;
+    while (__syncthreads_or(pending)) {
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+            if (rk[q] >= 0) atomicMin(M.bid + (t[q] & (kBidSlots - 1)), (uint32_t)rk[q]);
+        __syncthreads();
+        pending = false;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            if (rk[q] < 0) continue;
+            uint32_t *slot = M.bid + (t[q] & (kBidSlots - 1));
+            if (*(volatile uint32_t *)slot == (uint32_t)rk[q]) {
+                add(q);
+                *(volatile uint32_t *)slot = kNoBid;
+                rk[q] = -1;
+            } else {
+                pending = true;
+            }
+        }
+    }
 }
 
 // Neurons whose V this thread records after every step: it owns up to two observed
@@ -472,39 +544,13 @@ __device__ void sweep_network(const SweepDev &G, const SweepSmem &M, const Sweep
                 for (int p0 = 0;; p0 += cap) {
                     const int Sn = min(sources - p0, cap);
                     const int total = B.off[Sn];
-                    for (int e0 = 0; e0 < total; e0 += kBatch * nt) {
-                        uint16_t tq[kBatch];
-                        float wq[kBatch];
-                        int rk[kBatch];
-                        bool inh[kBatch];
-#pragma unroll
-                        for (int q = 0; q < kBatch; ++q) {
-                            const int e = e0 + q * nt + tid;
-                            rk[q] = -1;
-                            tq[q] = 0;
-                            wq[q] = 0.0f;
-                            inh[q] = false;
-                            if (e < total) {
-                                const int a = list_rank(B.off, Sn, e);
-                                const uint32_t o = B.base[a] + (uint32_t)(e - B.off[a]);
-                                tq[q] = __ldg(tg + o);
-                                wq[q] = __ldg(ww + o);
-                                const int x = B.src[a];
-                                inh[q] = x >= n_exc && x < n;
-                                rk[q] = a;
-                            }
-                        }
-                        const int r_lo = list_rank(B.off, Sn, e0);
-                        const int r_hi = list_rank(B.off, Sn, min(e0 + kBatch * nt, total) - 1);
-                        for (int a = r_lo; a <= r_hi; ++a) {
-#pragma unroll
-                            for (int q = 0; q < kBatch; ++q)
-                                if (rk[q] == a) {
-                                    float4 &x = M.x[tq[q] - first];
-                                    if (inh[q]) x.z += wq[q];
-                                    else x.y += wq[q];
-                                }
-                            __syncthreads();
+                    for (int e0 = 0; e0 < total;) {
+                        if (total - e0 <= nt) {
+                            deliver_batch<1>(M, B, Sn, e0, total, tg, ww, n_exc, n, first);
+                            e0 += nt;
+                        } else {
+                            deliver_batch<kBatch>(M, B, Sn, e0, total, tg, ww, n_exc, n, first);
+                            e0 += kBatch * nt;
                         }
                     }
                     if (tid == 0) events += (unsigned long long)total;
@@ -573,7 +619,9 @@ __global__ void __launch_bounds__(1024) k_sweep(SweepDev G, int nsteps, int max_
     SweepSmem M;
     M.x = reinterpret_cast<float4 *>(smem_raw);
     M.ring = reinterpret_cast<uint32_t *>(M.x + max_tile);
-    M.lists = reinterpret_cast<int32_t *>(M.ring + G.R * wc);
+    M.bid = M.ring + G.R * wc;
+    M.lists = reinterpret_cast<int32_t *>(M.bid + kBidSlots);
+    for (int x = threadIdx.x; x < kBidSlots; x += blockDim.x) M.bid[x] = kNoBid;  // (barriers follow before the first bid)
     M.cap = G.list_cap;
     __shared__ int s_net;
     __shared__ SweepLif s_L;

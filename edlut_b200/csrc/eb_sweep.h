@@ -16,6 +16,9 @@ using namespace eb;
 
 constexpr int kSweepMaxN = 16384;   // neurons per network
 constexpr int kSweepWindow = 8;     // steps between meetings of a network's CTAs and record drains
+constexpr int kRoundSources = 8;    // sources of a delivery batch from which it goes in rounds
+constexpr int kBidSlots = 1024;     // slots the rounds' entries bid for (a power of two)
+constexpr uint32_t kNoBid = 0xffffffffu;
 constexpr int64_t kDrainAtOnce = 1 << 20;  // spikes a drain copies without asking for their number first
 constexpr int kOwnObs = 1024;       // most observed neurons a network's threads record themselves
 constexpr int kTileMin = 256;       // fewest neurons a CTA of several per network is given

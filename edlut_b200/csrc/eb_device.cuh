@@ -51,8 +51,10 @@ struct Refr {
 
 // refr = updates since the last spike (-1: never spiked, LastSpikeTime >= 100 s).
 // LastSpikeTime = refr * dt exactly, because every partial sum of the reference's
-// double accumulation is exact.
-__device__ __forceinline__ Refr lif_refr(const PopDev &P, int refr) {
+// double accumulation is exact.  The host makes the reference's double comparisons once
+// per count (lif_refractory): in the update they were a chain of conversions and double
+// operations in every step.
+__host__ __device__ __forceinline__ Refr lif_refr_exact(const PopDev &P, int refr) {
     Refr r{0, 1.0f};
     if (refr < 0) return r;
     const double tref = (double)P.p[7];
@@ -65,6 +67,37 @@ __device__ __forceinline__ Refr lif_refr(const PopDev &P, int refr) {
         r.mode = 2;
     }
     return r;
+}
+
+__device__ __forceinline__ Refr lif_refr(const PopDev &P, int refr) {
+    if (P.ref_free < 0) return lif_refr_exact(P, refr);
+    Refr r{0, 1.0f};
+    if ((unsigned)refr < (unsigned)P.ref_free) {  // not the -1 of no spike yet
+        r.mode = refr < P.ref_part ? 2 : 1;
+        if (r.mode == 1) r.frac = P.ref_frac[refr - P.ref_part];
+    }
+    return r;
+}
+
+// Fill in ref_free, ref_part and ref_frac (host).
+inline void lif_refractory(PopDev &P) {
+    P.ref_part = -1;
+    for (int r = 0;; ++r) {
+        const Refr c = lif_refr_exact(P, r);
+        if (c.mode == 0) {
+            P.ref_free = r;
+            if (P.ref_part < 0) P.ref_part = r;
+            return;
+        }
+        if (c.mode == 1) {
+            if (P.ref_part < 0) P.ref_part = r;
+            if (r - P.ref_part >= 4) break;
+            P.ref_frac[r - P.ref_part] = c.frac;
+        } else if (P.ref_part >= 0 || r >= (1 << 24)) {
+            break;  // (not monotonic, or too long to tabulate)
+        }
+    }
+    P.ref_free = -1;
 }
 
 // x = {V, gE, gI, gNMDA}

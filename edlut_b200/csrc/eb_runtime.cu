@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "edlut_b200.h"
+#include "eb_device.cuh"
 #include "eb_kernels.h"
 #include "eb_record.h"
 #include "eb_runtime.h"
@@ -417,6 +418,7 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
             const float el = (p.integ == INTEG_RK4) ? D.dt_ms * 0.5f : D.dt_ms;  // RK4.h:362
             for (int c = 0; c < 3; ++c) D.decay[c] = decay_factor(el, tau[c]);
             bdf_coefficients(D.bdf_coef);
+            if (p.kind == KIND_LIF) lif_refractory(D);
             memcpy(D.init, init, sizeof(init));
             D.expt_aux = exp_table_aux();
             D.exp_table = N.exp_table;

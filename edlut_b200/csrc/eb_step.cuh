@@ -584,7 +584,7 @@ struct NarrowStage {
 __host__ __device__ constexpr int narrow_stage(int kind) { return kind == KIND_HH ? 128 : 64; }
 static_assert(kMaxWindow <= 8, "a lane packs a window's counts into 8 bytes");
 
-template <int KIND, int INTEG, int EN, int MON, bool SMALL, int CAP>
+template <int KIND, int INTEG, int EN, int MON, bool SMALL, bool PLASTIC, int CAP>
 __device__ __forceinline__ void narrow_window(const PopDev &P, const NetDev &N, int64_t k, int64_t i, bool active,
                                               float *x, NeuronAux &ax, int nsteps, double push_inv_dt,
                                               NarrowStage<CAP> &S) {
@@ -592,7 +592,7 @@ __device__ __forceinline__ void narrow_window(const PopDev &P, const NetDev &N, 
     constexpr unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t gi = P.first + i;
-    const bool plastic = P.post_t != nullptr;
+    constexpr bool plastic = PLASTIC;
     // counts of the steps not yet run, a byte each (255: that many or more), next step lowest
     unsigned long long pk = 0;
     uint32_t capg = 0;
@@ -739,6 +739,8 @@ __device__ __forceinline__ void narrow_window(const PopDev &P, const NetDev &N, 
 
 // Steps k .. k+nsteps-1 of one tile, the state in registers between them.
 // push_inv_dt > 0: also fan out the spikes (1 / step, for arrival_step).
+// PLASTIC: the population keeps a post-synaptic spike ring; the staged window of one that
+// does not is half the code, and a warp alone on its sub-partition waits for code.
 // SMALL: registers are not bounded and a warp keeps more accesses of a fan-out in
 // flight (populations that fit the SMs all the same, see eb_update.cu).
 // HH under BDF holds the Newton state (Jacobian, inverse, history) in about 120
@@ -753,7 +755,7 @@ constexpr int narrow_min_blocks(int kind, int integ) {
     return (kind == KIND_HH && integ == INTEG_BDF) ? 3 : (kind != KIND_HH && integ != INTEG_BDF) ? 5 : 0;
 }
 
-template <int KIND, int INTEG, int EN, int MON, bool SMALL>
+template <int KIND, int INTEG, int EN, int MON, bool SMALL, bool PLASTIC>
 __global__ void __launch_bounds__(kNarrowBlock, SMALL ? 1 : narrow_min_blocks(KIND, INTEG) * (kNarrowTile / kNarrowBlock)) k_update_narrow(PopDev P, NetDev N, int rel, int nsteps,
                                                                 double push_inv_dt, int npw) {
     const int64_t k = cur_step(N, rel);
@@ -768,7 +770,7 @@ __global__ void __launch_bounds__(kNarrowBlock, SMALL ? 1 : narrow_min_blocks(KI
         ax = load_aux<KIND, INTEG>(P, i);
     }
     if constexpr (SMALL || KIND == KIND_HH) {
-        narrow_window<KIND, INTEG, EN, MON, SMALL>(P, N, k, i, active, x, ax, nsteps, push_inv_dt, stage[threadIdx.x >> 5]);
+        narrow_window<KIND, INTEG, EN, MON, SMALL, PLASTIC>(P, N, k, i, active, x, ax, nsteps, push_inv_dt, stage[threadIdx.x >> 5]);
     } else {
         for (int s = 0; s < nsteps; ++s)
             narrow_step<KIND, INTEG, EN, MON>(P, N, k + s, i, active, x, ax, false, push_inv_dt);

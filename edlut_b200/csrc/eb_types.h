@@ -81,6 +81,11 @@ struct PopDev {
     float dt_s, dt_ms;
     float inv_c_m, inv_slope, inv_tau_w;
     float adex_vmax, adex_glslope;  // AdEx: vthr + 6 * slope, gl * slope
+    // LIF refractoriness by updates since the last spike: free from ref_free on, a fraction
+    // ref_frac[refr - ref_part] of the derivative from ref_part on, none before; ref_free
+    // is -1 when the period has more fractional steps than ref_frac holds
+    int ref_free, ref_part;
+    float ref_frac[4];
     float decay[3];  // conductance decay factor per step (RK4: per half step)
     float bdf_coef[7][7];
     float init[kMaxVars];

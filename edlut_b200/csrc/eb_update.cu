@@ -36,11 +36,15 @@ void launch_update_t(const PopDev &P, const NetDev &N, int rel, int nsteps, doub
         const int npw = narrow_npw(P.n), tile = narrow_tile(npw), per = tile / 32 * npw;
         const int blocks = (int)((P.n + per - 1) / per);
         auto launch = [&](auto fn) { fn<<<blocks, tile, 0, st>>>(P, N, rel, nsteps, push_inv_dt, npw); };
-        const bool small = P.n <= narrow_few(KIND);
-        if (P.mon) launch(k_update_narrow<KIND, INTEG, -1, 1, true>);
-        else if (P.en == 1) small ? launch(k_update_narrow<KIND, INTEG, 1, 0, true>) : launch(k_update_narrow<KIND, INTEG, 1, 0, false>);
-        else if (P.en == 3) small ? launch(k_update_narrow<KIND, INTEG, 3, 0, true>) : launch(k_update_narrow<KIND, INTEG, 3, 0, false>);
-        else launch(k_update_narrow<KIND, INTEG, -1, 0, false>);
+        // the per-step fold of large populations asks at run time: its code is the same
+        const bool small = P.n <= narrow_few(KIND), plastic = P.post_t != nullptr, staged = small || KIND == KIND_HH;
+        if (P.mon) plastic ? launch(k_update_narrow<KIND, INTEG, -1, 1, true, true>) : launch(k_update_narrow<KIND, INTEG, -1, 1, true, false>);
+        else if (P.en == 1 && small) plastic ? launch(k_update_narrow<KIND, INTEG, 1, 0, true, true>) : launch(k_update_narrow<KIND, INTEG, 1, 0, true, false>);
+        else if (P.en == 3 && small) plastic ? launch(k_update_narrow<KIND, INTEG, 3, 0, true, true>) : launch(k_update_narrow<KIND, INTEG, 3, 0, true, false>);
+        else if (staged && plastic) launch(k_update_narrow<KIND, INTEG, -1, 0, false, true>);
+        else if (P.en == 1) launch(k_update_narrow<KIND, INTEG, 1, 0, false, false>);
+        else if (P.en == 3) launch(k_update_narrow<KIND, INTEG, 3, 0, false, false>);
+        else launch(k_update_narrow<KIND, INTEG, -1, 0, false, false>);
     }
 }
 

@@ -295,7 +295,7 @@ __device__ __forceinline__ bool advance_neuron(const PopDev &P, const NetDev &N,
         if (KIND == KIND_LIF) refr = 0;  // NewFiredSpike
         if (reset && INTEG == INTEG_BDF) bst = 0;
     }
-    if (x[0] != x[0]) {  // CheckValidIntegration: reset a neuron whose V became NaN
+    if (__builtin_expect(x[0] != x[0], 0)) {  // CheckValidIntegration: reset a neuron whose V became NaN
 #pragma unroll
         for (int v = 0; v < NV; ++v) x[v] = P.init[v];
     }
@@ -593,6 +593,8 @@ __device__ __forceinline__ void narrow_window(const PopDev &P, const NetDev &N, 
     const int lane = threadIdx.x & 31;
     const int64_t gi = P.first + i;
     constexpr bool plastic = PLASTIC;
+    const bool fan_out = push_inv_dt > 0.0;
+    const bool traced = N.trace && gi >= N.trace_first && gi < N.trace_first + N.trace_n;
     // counts of the steps not yet run, a byte each (255: that many or more), next step lowest
     unsigned long long pk = 0;
     uint32_t capg = 0;
@@ -728,12 +730,14 @@ __device__ __forceinline__ void narrow_window(const PopDev &P, const NetDev &N, 
             }
             pos += c;
             sp = advance_neuron<KIND, INTEG, EN>(P, N, i, x, ax);
-            record_trace(P, N, ks, gi, x, Model<KIND>::NV);
+            if (traced) record_trace(P, N, ks, gi, x, Model<KIND>::NV);
             if (mon_on<MON>(P)) monitor_state(P, N, ks, i, x, Model<KIND>::NV, sp);
             if (sp && plastic) note_post_spike(P, N, i, ks);
         }
-        compact_spikes(P, N, ks, i, sp, false);
-        if (push_inv_dt > 0.0) warp_push<SMALL ? 4 : 1>(P, N, ks, i, sp, push_inv_dt);
+        if (__any_sync(full, sp)) {
+            compact_spikes(P, N, ks, i, sp, false);
+            if (fan_out) warp_push<SMALL ? 4 : 1>(P, N, ks, i, sp, push_inv_dt);
+        }
     }
 }
 

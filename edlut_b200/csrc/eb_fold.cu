@@ -225,10 +225,17 @@ extern "C" int eb_fold_arrivals(void *stream, int64_t n, const int32_t *target, 
     void *scratch = nullptr;
     const size_t bytes = fold_scratch_bytes(n, n_targets);
     if (n == 0) return EB_OK;
-    cudaMemPool_t pool;
-    if ((rc = fold_pool(&pool))) return rc;
-    cudaError_t e = cudaMallocFromPoolAsync(&scratch, bytes, pool, st);
-    if (e != cudaSuccess) { set_error("cudaMallocFromPoolAsync(%zu): %s", bytes, cudaGetErrorString(e)); return EB_ERR_NOMEM; }
+    // under stream capture the scratch is a node of the graph, which owns it
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &capture);
+    cudaMemPool_t pool = nullptr;
+    if (e == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        if ((rc = fold_pool(&pool))) return rc;
+        e = cudaMallocFromPoolAsync(&scratch, bytes, pool, st);
+    } else if (e == cudaSuccess) {
+        e = cudaMallocAsync(&scratch, bytes, st);
+    }
+    if (e != cudaSuccess) { set_error("fold scratch (%zu bytes): %s", bytes, cudaGetErrorString(e)); return EB_ERR_NOMEM; }
     rc = fold_enqueue(st, scratch, n, target, type, weight, time, n_targets, g_exc, g_inh, g_nmda);
     cudaFreeAsync(scratch, st);
     return rc;

@@ -87,6 +87,13 @@ static int upload(eb_ctx *c, T **dptr, const std::vector<T> &h) {
     return EB_OK;
 }
 
+// The weights' staging buffer: with the network when it learns (its weights are read),
+// else on first use.
+int eb_ctx::ensure_wstage() {
+    if (d_wstage || src.empty()) return EB_OK;
+    return dalloc((void **)&d_wstage, sizeof(float) * (size_t)std::min<int64_t>((int64_t)src.size(), kWeightChunk));
+}
+
 // ----------------------------------------------------------- construction --
 int eb_ctx::add_population(int kind, int64_t n, int integ, int bdf_order, float dt, const float *params,
                            int n_params, int64_t *out_first) {
@@ -492,6 +499,7 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
         }
         D.may_repeat = in_from_inputs > 0 ? 1 : 0;
     }
+    if (lazy_post && (rc = ensure_wstage())) return rc;
     plan_chains(out_ptr, h_out_tgt, h_out_units);
     if ((rc = seed_generators())) return rc;
     // dynamic state copied by eb_snapshot / eb_restore
@@ -1549,7 +1557,7 @@ static int weights_io(eb_ctx *ctx, float *w, bool get) {
     if ((rc = ctx->flush_post())) return rc;
     const int64_t m = (int64_t)ctx->src.size();
     const int64_t chunk = std::min<int64_t>(m, kWeightChunk);
-    if (m && !ctx->d_wstage && (rc = ctx->dalloc((void **)&ctx->d_wstage, sizeof(float) * (size_t)chunk))) return rc;
+    if ((rc = ctx->ensure_wstage())) return rc;
     for (int64_t k = 0; k < m; k += chunk) {
         const int64_t c = std::min(chunk, m - k);
         if (get) {

@@ -69,7 +69,7 @@ struct eb_ctx {
     int R = 0;
     std::vector<int> pop_of;
     uint32_t *d_tpos = nullptr;   // file order -> target-major position of each synapse
-    float *d_wstage = nullptr;    // weights on their way to or from the host (first use)
+    float *d_wstage = nullptr;    // weights on their way to or from the host (ensure_wstage)
     eb::NetDev net{};
     int64_t *d_step = nullptr;
     eb::RunStatus *status = nullptr;  // pinned, written by the device at the end of each run segment
@@ -154,6 +154,7 @@ struct eb_ctx {
     struct HostSnap { int slot; int64_t steps_done, spikes_drained; int steps_since_flush; };
     std::vector<HostSnap> snap_host;
 
+    int ensure_wstage();
     int dalloc(void **p, size_t bytes);
     void dfree(void *p);
     void dfree_all();

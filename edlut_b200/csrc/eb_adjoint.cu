@@ -37,6 +37,7 @@ using namespace ebsw;
 
 namespace {
 
+constexpr int kAhead = 4;       // steps whose trajectory k_adj_neuron loads ahead
 constexpr int kInstCap = 4096;  // spike instances per weight-gradient pass
 
 // Adjoint of one derivative evaluation D(V, gE, gI) (sw_deriv): lk = dL/dD.
@@ -143,7 +144,7 @@ __device__ __forceinline__ float frac_of(const SweepLif &L, int fi) {
 // the parameter partials in gacc (double, per neuron) and writes the adjoint of
 // each step's post-arrival conductances to muE / muI for the weight gradients.
 template <int INTEG>
-__global__ void __launch_bounds__(256) k_adj_neuron(SweepDev G, const SweepNet *nets, int64_t k_lo, int len,
+__global__ void __launch_bounds__(128) k_adj_neuron(SweepDev G, const SweepNet *nets, int64_t k_lo, int len,
                                                      int64_t n_steps, const float *gtrace, const int32_t *obs_slot,
                                                      float *lamV, float *lamE, float *lamI, double *gacc, float *muE,
                                                      float *muI, int first_seg) {
@@ -158,29 +159,54 @@ __global__ void __launch_bounds__(256) k_adj_neuron(SweepDev G, const SweepNet *
     const float dt = G.dt_ms;
     float lV = lamV[gi], lE = lamE[gi], lI = lamI[gi];
     double aGL = 0.0, aEL = 0.0, aAE = 0.0, aAI = 0.0;
-    for (int kk = len - 1; kk >= 0; --kk) {
+    // The trajectory of kAhead steps is on its way while one is worked on: a thread's steps
+    // are serial, but their inputs are not, and there are few warps to hide the loads.
+    struct Inputs {
+        float V, gE, gI, g;
+        int code;
+    };
+    auto load = [&](int kk) {
         const int64_t x = (int64_t)kk * Nt + gi;
-        if (m >= 0) lV += gtrace[((int64_t)net * n_steps + (k_lo + kk)) * G.n_obs + m];
-        const int code = G.tcode[x];
-        const float V = G.tV[x], gE = G.tE[x], gI = G.tI[x];
-        const int cls = code & 3;
-        const float f = cls == 2 ? frac_of(L, (code >> 2) & 3) : 1.0f;
-        float pGL = 0.0f, pEL = 0.0f, pAE = 0.0f, pAI = 0.0f;
-        if (code & kCodeSpike) {  // V_k = E_leak: the jump cuts lambda_V
-            aEL += (double)lV;
-            lV = 0.0f;
+        Inputs v;
+        v.V = __ldg(G.tV + x);
+        v.gE = __ldg(G.tE + x);
+        v.gI = __ldg(G.tI + x);
+        v.code = __ldg(G.tcode + x);
+        v.g = m >= 0 ? __ldg(gtrace + ((int64_t)net * n_steps + (k_lo + kk)) * G.n_obs + m) : 0.0f;
+        return v;
+    };
+    Inputs buf[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+        if (len - 1 - u >= 0) buf[u] = load(len - 1 - u);
+    for (int k1 = len - 1; k1 >= 0; k1 -= kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int kk = k1 - u;
+            if (kk < 0) break;
+            const Inputs in = buf[u];
+            if (kk >= kAhead) buf[u] = load(kk - kAhead);
+            if (m >= 0) lV += in.g;
+            const int cls = in.code & 3;
+            const float f = cls == 2 ? frac_of(L, (in.code >> 2) & 3) : 1.0f;
+            float pGL = 0.0f, pEL = 0.0f, pAE = 0.0f, pAI = 0.0f;
+            if (in.code & kCodeSpike) {  // V_k = E_leak: the jump cuts lambda_V
+                aEL += (double)lV;
+                lV = 0.0f;
+            }
+            float nV, nE, nI;
+            d_integrate<INTEG>(L, dt, in.V, in.gE, in.gI, cls, f, lV, lE, lI, nV, nE, nI, pGL, pEL, pAE, pAI);
+            lV = nV;
+            lE = nE;
+            lI = nI;
+            const int64_t x = (int64_t)kk * Nt + gi;
+            muE[x] = lE;
+            muI[x] = lI;
+            aGL += (double)pGL;
+            aEL += (double)pEL;
+            aAE += (double)pAE;
+            aAI += (double)pAI;
         }
-        float nV, nE, nI;
-        d_integrate<INTEG>(L, dt, V, gE, gI, cls, f, lV, lE, lI, nV, nE, nI, pGL, pEL, pAE, pAI);
-        lV = nV;
-        lE = nE;
-        lI = nI;
-        muE[x] = lE;
-        muI[x] = lI;
-        aGL += (double)pGL;
-        aEL += (double)pEL;
-        aAE += (double)pAE;
-        aAI += (double)pAI;
     }
     if (first_seg) aEL += (double)lV;  // V_0 = E_leak
     lamV[gi] = lV;
@@ -324,22 +350,20 @@ __global__ void __launch_bounds__(256) k_adj_wgrad(SweepDev G, const SweepNet *n
     }
 }
 
-// Per-network sums of the per-neuron partials, in a fixed order.
+// Per-network sums of the per-neuron partials, in a fixed order: block (network, partial).
 __global__ void k_adj_reduce(const SweepNet *nets, int64_t Nt, const double *gacc, double *out) {
     __shared__ double sh[256];
     const SweepNet &S = nets[blockIdx.x];
-    for (int c = 0; c < 4; ++c) {
-        double a = 0.0;
-        for (int i = threadIdx.x; i < S.n; i += blockDim.x) a += gacc[c * Nt + S.state_off + i];
-        sh[threadIdx.x] = a;
-        __syncthreads();
-        for (int st = blockDim.x >> 1; st > 0; st >>= 1) {
-            if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[blockIdx.x * 4 + c] = sh[0];
+    const int c = blockIdx.y;
+    double a = 0.0;
+    for (int i = threadIdx.x; i < S.n; i += blockDim.x) a += gacc[c * Nt + S.state_off + i];
+    sh[threadIdx.x] = a;
+    __syncthreads();
+    for (int st = blockDim.x >> 1; st > 0; st >>= 1) {
+        if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
         __syncthreads();
     }
+    if (threadIdx.x == 0) out[blockIdx.x * 4 + c] = sh[0];
 }
 
 __global__ void __launch_bounds__(256) k_adj_obs(SweepDev G, const SweepNet *nets, int32_t *obs_slot) {
@@ -433,15 +457,18 @@ extern "C" int eb_sweep_adjoint(eb_sweep *h, const float *grad_trace, int gt_on_
     k_adj_clear<<<148 * 4, 256, 0, st>>>(Nt, h->lamV, h->lamE, h->lamI, h->gacc, h->total_syn, h->gw_sorted, h->G.flags);
     SK(cudaGetLastError());
     const AdjFn fa = adj_fn(h->integ);
-    const dim3 ga((h->max_n + 255) / 256, h->n_nets);
-    const int parts = std::max(1, (2 * 148 + h->n_nets - 1) / h->n_nets);
+    const dim3 ga((h->max_n + 127) / 128, h->n_nets);
+    // source ranges per network: k_adj_wgrad waits for dependent loads (range -> target ->
+    // adjoint), so each block takes few sources and many blocks are resident (8 networks of
+    // up to 10,000 neurons, a fitting step: 2 blocks an SM 7.29 ms, 6 7.22, 12 7.06)
+    const int parts = std::max(1, (12 * 148 + h->n_nets - 1) / h->n_nets);
     const std::vector<int32_t> &arr = h->h_arr_step;
     for (int s = nseg - 1; s >= 0; --s) {
         const int64_t k_lo = (int64_t)s * E;
         const int len = (int)std::min<int64_t>(E, S - k_lo);
         if ((rc = checkpoint_restore(h, s, k_lo, st))) break;
         if ((rc = enqueue_chunk(h, len, st, true, k_lo))) break;
-        fa<<<ga, 256, 0, st>>>(h->G, h->d_nets, k_lo, len, S, gt, h->obs_slot, h->lamV, h->lamE, h->lamI, h->gacc,
+        fa<<<ga, 128, 0, st>>>(h->G, h->d_nets, k_lo, len, S, gt, h->obs_slot, h->lamV, h->lamE, h->lamI, h->gacc,
                                h->muE, h->muI, s == 0 ? 1 : 0);
         // source steps whose spikes arrive in the segment
         const int32_t k1 = (int32_t)(k_lo + 1), k2 = (int32_t)(k_lo + len);
@@ -455,7 +482,7 @@ extern "C" int eb_sweep_adjoint(eb_sweep *h, const float *grad_trace, int gt_on_
     if (gt_tmp) cudaFreeAsync(gt_tmp, st);
     h->needs_reset = true;
     if (rc) return rc;
-    k_adj_reduce<<<h->n_nets, 256, 0, st>>>(h->d_nets, Nt, h->gacc, h->red_out);
+    k_adj_reduce<<<dim3(h->n_nets, 4), 256, 0, st>>>(h->d_nets, Nt, h->gacc, h->red_out);
     SK(cudaGetLastError());
     if (grad_w && h->total_syn) {
         float *dst = grad_w, *tmp = nullptr;

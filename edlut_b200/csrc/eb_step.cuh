@@ -1409,8 +1409,8 @@ __device__ __forceinline__ void wide_window(const PopDev &P, const NetDev &N, in
 
 // Steps k .. k+nsteps-1 of the block's neurons.
 // Populations whose synapses cannot deliver twice in one step take the staged
-// window; the others run step by step.  At most 72 registers a thread: three
-// blocks per SM leave room for one thread-per-neuron block of 256 at 40.
+// window; the others run step by step.  At most 72 registers a thread: blocks of
+// this kernel share an SM with the thread-per-neuron blocks of 256 (48 registers).
 template <int KIND, int INTEG, int MON, int EN>
 __global__ void __maxnreg__(72) k_update_wide(PopDev P, NetDev N, int rel, int nsteps,
                                                                  double push_inv_dt) {

@@ -979,11 +979,9 @@ int eb_sweep_build(eb_sweep *h, int64_t n_steps_max, float max_rate_hz) {
             lag = std::min(lag, ka - j);
         }
     }
-    // A window's sources precede it (at most `lag` steps, the fewest from a spike to its
-    // arrival); the ring holds the sources of its lists, then the spikes of the window
-    // being drained, while the next window's are written.
-    h->G.window = (int)std::max<int64_t>(1, std::min<int64_t>(kSweepWindow, lag));
-    const int R = (int)dmax + 1 + h->G.window;
+    const SweepRing ring = sweep_ring(dmax, lag);
+    const int R = ring.slots;
+    h->G.window = ring.window;
     h->G.R = R;
     h->G.steps_max = (int)n_steps_max;
     h->G.dt_ms = h->dt * 1000.0f;

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -25,6 +26,20 @@ constexpr int kTileMin = 256;       // fewest neurons a CTA of several per netwo
 constexpr int kBatch = 4;           // synapses per thread per delivery batch
 constexpr int kMaxGroups = 3;       // source steps arriving in one step
 constexpr int kMaxFrac = 4;         // steps with a partial refractory fraction
+
+// Steps of a window and slots of the delay ring, from the most and fewest steps between a
+// spike and its arrival (most 1, fewest above any window where nothing arrives at all).
+// A window's sources precede it, so it is no longer than the fewest.  The ring holds the
+// sources of a window's lists (`most` steps and the one being listed) or the window being
+// drained, whichever is more, and beside them the window that the network's other CTAs
+// write in the meantime.
+struct SweepRing {
+    int window, slots;
+};
+inline SweepRing sweep_ring(int64_t most, int64_t fewest) {
+    const int64_t w = std::max<int64_t>(1, std::min<int64_t>(kSweepWindow, fewest));
+    return {(int)w, (int)(std::max(most + 1, w) + w)};
+}
 
 // Per neuron-step trajectory code: bits 0-1 refractory class (0 none, 1 frozen,
 // 2 fraction), bits 2-3 fraction index, bit 4 spike.

@@ -172,3 +172,24 @@ def test_sweeps_of_different_sizes_live_side_by_side():
     assert_network_matches(small, 7, nsteps)
     big.close()
     small.close()
+
+
+@pytest.mark.parametrize("n,nsteps", [(520, 40), (2050, 40), (2050, 49)])
+def test_clustered_run_shorter_than_its_delay_matches_solo_runs(n, nsteps):
+    # no spike arrives within the run (5 ms are 50 steps), and every neuron fires in every
+    # step: the CTAs of a network meet only once a window, while the first one drains it
+    specs = sweep_networks(seed=n, n_networks=2, n_min=n, n_max=n + 40, t_end=nsteps * 1e-4)
+    for s in specs:
+        s["params"]["e_leak"] = -45.0
+    sw = make_sweep(specs, nsteps, max_rate_hz=10000.0, delay=5e-3)
+    want = [solo(sw, i, nsteps) for i in range(len(specs))]
+    for _ in range(30):
+        sw.reset()
+        sw.run(nsteps)
+        for i, (st, ce, v) in enumerate(want):
+            s2, c2 = sw.spikes(i)
+            np.testing.assert_array_equal(st, s2)
+            np.testing.assert_array_equal(ce, c2)
+            np.testing.assert_array_equal(v, sw.state(i, 0))
+        np.testing.assert_array_equal(sw.spike_counts(), [len(w[0]) for w in want])
+    sw.close()

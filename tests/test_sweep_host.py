@@ -1,5 +1,10 @@
-"""CPU tests of the sweep workload generator (no GPU)."""
+"""CPU tests of the sweep workload generator and of the delay ring's size (no GPU)."""
+import os
+import shutil
+import subprocess
+
 import numpy as np
+import pytest
 
 from edlut_b200.configs import LIF_C1, sweep_networks
 
@@ -30,3 +35,49 @@ def test_sweep_weight_scaling_keeps_mean_drive():
         # recurrent range x size / 1000 is the weight-scale factor, the same as the input range's
         k = s["w_exc_max"] * s["n"] / 1000.0 / 0.5
         assert abs(k - s["w_in_max"] / 0.5) < 1e-4 * max(1.0, k)
+
+
+# The rows of a network's ring that are in use at once must have slots of their own: while
+# one CTA still drains window w (or lists the sources of window w + 1), the others already
+# write window w + 1.
+RING_PROGRAM = r"""
+#include <cstdio>
+#include <set>
+#include "eb_sweep.h"
+int main() {
+    long bad = 0;
+    auto check = [&](int64_t most, int64_t fewest, bool arrives) {
+        const ebsw::SweepRing r = ebsw::sweep_ring(most, fewest);
+        bad += r.window < 1 || r.window > ebsw::kSweepWindow || r.window > fewest;
+        const int64_t kw = 1000;  // first step of window w
+        std::set<int64_t> rows;
+        for (int64_t k = kw; k < kw + 2 * r.window; ++k) rows.insert(k);  // drained, written
+        if (arrives)  // sources of window w + 1's lists
+            for (int64_t k = kw + r.window; k < kw + 2 * r.window; ++k)
+                for (int64_t j = k - most; j <= k - fewest; ++j) rows.insert(j);
+        std::set<int64_t> slots;
+        for (int64_t k : rows) slots.insert(k % r.slots);
+        bad += slots.size() != rows.size();
+    };
+    for (int64_t fewest = 1; fewest <= 40; ++fewest)
+        for (int64_t most = fewest; most <= fewest + 3; ++most) check(most, fewest, true);
+    check(1, INT32_MAX, false);  // no spike arrives within the run
+    printf("%ld\n", bad);
+}
+"""
+
+
+@pytest.mark.skipif(not shutil.which("g++"), reason="needs g++")
+def test_ring_keeps_a_window_apart_from_the_one_being_drained(tmp_path):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src = tmp_path / "ring.cpp"
+    src.write_text(RING_PROGRAM)
+    exe = str(tmp_path / "ring")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    if not os.path.exists(os.path.join(cuda, "include", "cuda_runtime.h")):
+        pytest.skip("needs the CUDA headers")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-I" + os.path.join(root, "edlut_b200", "csrc"),
+                    "-I" + os.path.join(root, "include"), "-I" + os.path.join(cuda, "include"), str(src), "-o", exe,
+                    "-L" + os.path.join(cuda, "lib64"), "-lcudart"], check=True)
+    out = subprocess.run([exe], capture_output=True, text=True, check=True).stdout
+    assert int(out) == 0

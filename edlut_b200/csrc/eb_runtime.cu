@@ -343,21 +343,21 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
     CK(cudaMemsetAsync(N.rec_count, 0, sizeof(unsigned long long), st));
     N.rec_cap = rec_cap;
     if (rec_cap > 0 && (rc = dalloc((void **)&N.rec_buf, sizeof(unsigned long long) * (size_t)rec_cap))) return rc;
-    has_inputs = false;
-    for (auto &p : pops)
-        if (p.kind == KIND_INPUT) has_inputs = true;
-    // input fan-out may run beside the neuron updates when no input delivery can
-    // reach the step being updated: every input synapse delay exceeds the step
-    {
-        int64_t min_units = INT64_MAX, max_out_in = 0;
-        for (int64_t i = 0; i < n_neurons; ++i) {
-            if (pops[pop_of[i]].kind != KIND_INPUT) continue;
-            max_out_in = std::max(max_out_in, out_ptr[i + 1] - out_ptr[i]);
-            for (int64_t s = out_ptr[i]; s < out_ptr[i + 1]; ++s) min_units = std::min<int64_t>(min_units, h_out_units[s]);
+    const size_t np = pops.size();
+    pair_delay.assign(np * np, PairDelay{});
+    max_out.assign(np, 0);
+    for (int64_t i = 0; i < n_neurons; ++i) {
+        const size_t a = (size_t)pop_of[i];
+        max_out[a] = std::max(max_out[a], out_ptr[i + 1] - out_ptr[i]);
+        for (int64_t s = out_ptr[i]; s < out_ptr[i + 1]; ++s) {
+            PairDelay &d = pair_delay[a * np + (size_t)pop_of[h_out_tgt[s]]];
+            d.lo = std::min<int64_t>(d.lo, h_out_units[s]);
+            d.hi = std::max<int64_t>(d.hi, h_out_units[s]);
         }
-        inputs_concurrent = min_units == INT64_MAX || (double)min_units * 0.0001 > dt_s;
-        input_threads = (int)std::min<int64_t>(256, std::max<int64_t>(32, (max_out_in + 31) / 32 * 32));
     }
+    feeds.assign(np, 0);
+    for (size_t q = 0; q < np; ++q) feeds[q] = pops[q].kind == KIND_INPUT;
+    for (const auto &p : pending) feeds[pop_of[p.cell]] = 1;
     net = N;
 
     // populations
@@ -492,15 +492,12 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
             D.post_rule = -1;
         }
         p.has_out = false;
-        int64_t in_from_inputs = 0;
-        for (int64_t i = p.first; i < p.first + p.n; ++i) {
+        for (int64_t i = p.first; i < p.first + p.n; ++i)
             if (out_ptr[i + 1] > out_ptr[i]) p.has_out = true;
-            in_from_inputs += indeg_in[i];
-        }
-        D.may_repeat = in_from_inputs > 0 ? 1 : 0;
     }
     if (lazy_post && (rc = ensure_wstage())) return rc;
-    plan_chains(out_ptr, h_out_tgt, h_out_units);
+    plan_inputs();
+    plan_chains();
     if ((rc = seed_generators())) return rc;
     // dynamic state copied by eb_snapshot / eb_restore
     dyn.clear();
@@ -529,18 +526,7 @@ int eb_ctx::finalize(int64_t *out_sorted_perm) {
             if (p.dev.post_f) dyn.push_back({p.dev.post_f, sizeof(DecayPair) * (size_t)kPostRing * p.n});
         }
     }
-    for (int q = 0; q < std::max(4, (int)chain_pop.size() - 1); ++q) {
-        cudaStream_t ss;
-        CK(cudaStreamCreateWithFlags(&ss, cudaStreamNonBlocking));
-        side.push_back(ss);
-    }
-    for (int q = 0; q < std::max(8, (int)chain_pop.size()); ++q) {
-        cudaEvent_t a, b;
-        CK(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&b, cudaEventDisableTiming));
-        fork_ev.push_back(a);
-        join_ev.push_back(b);
-    }
+    if ((rc = ensure_chain_streams())) return rc;
     if ((rc = setup_persistent())) return rc;
     CK(prepare_update_kernels());
     CK(cudaStreamSynchronize(st));
@@ -877,6 +863,61 @@ int eb_ctx::setup_persistent() {
     return EB_OK;
 }
 
+// What depends on the populations that input spikes enter (feeds).
+void eb_ctx::plan_inputs() {
+    const size_t np = pops.size();
+    has_inputs = false;
+    // input fan-out may run beside the neuron updates when no input delivery can
+    // reach the step being updated: every input synapse delay exceeds the step
+    int64_t min_units = INT64_MAX, most = 0;
+    for (size_t b = 0; b < np; ++b) pops[b].dev.may_repeat = 0;
+    for (size_t a = 0; a < np; ++a) {
+        if (!feeds[a]) continue;
+        has_inputs = true;
+        most = std::max(most, max_out[a]);
+        for (size_t b = 0; b < np; ++b) {
+            if (pair_delay[a * np + b].hi < 0) continue;
+            min_units = std::min(min_units, pair_delay[a * np + b].lo);
+            pops[b].dev.may_repeat = 1;
+        }
+    }
+    inputs_concurrent = min_units == INT64_MAX || (double)min_units * 0.0001 > dt_s;
+    input_threads = (int)std::min<int64_t>(256, std::max<int64_t>(32, (most + 31) / 32 * 32));
+    pinfo.has_inputs = has_inputs ? 1 : 0;
+    pinfo.inputs_concurrent = inputs_concurrent ? 1 : 0;
+}
+
+// Streams and events of the plan's chains and of a step's branches.
+int eb_ctx::ensure_chain_streams() {
+    const int nc = (int)chain_pop.size();
+    while ((int)side.size() < std::max(4, nc - 1)) {
+        cudaStream_t ss;
+        CK(cudaStreamCreateWithFlags(&ss, cudaStreamNonBlocking));
+        side.push_back(ss);
+    }
+    while ((int)fork_ev.size() < std::max(8, nc)) {
+        cudaEvent_t a, b;
+        CK(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
+        fork_ev.push_back(a);
+        CK(cudaEventCreateWithFlags(&b, cudaEventDisableTiming));
+        join_ev.push_back(b);
+    }
+    return EB_OK;
+}
+
+// Input spikes enter model population q from now on (finalized network): its synapses may
+// deliver twice in a step, and its targets' updates wait for the input fan-out too.
+int eb_ctx::feed_population(int q) {
+    if (feeds[q]) return EB_OK;
+    CK(cudaSetDevice(device));
+    feeds[q] = 1;
+    graphs_valid = false;
+    pops_dirty = true;
+    plan_inputs();
+    plan_chains();
+    return ensure_chain_streams();
+}
+
 // Chains of the captured graph: one per model population, one for all input
 // neurons (chain 0, so that its launch of step r is captured before the updates of
 // step r).  Population B's update at step k reads and clears bucket slot k; a
@@ -895,27 +936,30 @@ int eb_ctx::setup_persistent() {
 // hi), its own population's included, is at least S.  Input chains may feed a
 // window of the same index (lo < S): they are captured first and wait for nothing
 // of that window.
-void eb_ctx::plan_chains(const std::vector<int64_t> &out_ptr, const std::vector<uint32_t> &out_tgt,
-                         const std::vector<uint16_t> &out_units) {
+void eb_ctx::plan_chains() {
     chain_pop.clear();
     chain_deps.clear();
-    std::vector<int> chain_of(pops.size(), -1);
+    const size_t np = pops.size();
+    std::vector<int> chain_of(np, -1);
     if (has_inputs) chain_pop.push_back(-1);
-    for (size_t q = 0; q < pops.size(); ++q) {
+    for (size_t q = 0; q < np; ++q) {
         if (pops[q].kind == KIND_INPUT) chain_of[q] = 0;
         else { chain_of[q] = (int)chain_pop.size(); chain_pop.push_back((int)q); }
     }
     const int nc = (int)chain_pop.size();
     std::vector<int64_t> umin((size_t)nc * nc, INT64_MAX), umax((size_t)nc * nc, -1);
-    for (int64_t i = 0; i < n_neurons; ++i) {
-        const int a = chain_of[pop_of[i]];
-        for (int64_t s = out_ptr[i]; s < out_ptr[i + 1]; ++s) {
-            const int b = chain_of[pop_of[out_tgt[s]]];
-            const size_t e = (size_t)a * nc + b;
-            umin[e] = std::min<int64_t>(umin[e], out_units[s]);
-            umax[e] = std::max<int64_t>(umax[e], out_units[s]);
+    for (size_t a = 0; a < np; ++a)
+        for (size_t b = 0; b < np; ++b) {
+            const PairDelay &d = pair_delay[a * np + b];
+            if (d.hi < 0) continue;
+            const auto edge = [&](int from) {
+                const size_t e = (size_t)from * nc + chain_of[b];
+                umin[e] = std::min(umin[e], d.lo);
+                umax[e] = std::max(umax[e], d.hi);
+            };
+            edge(chain_of[a]);
+            if (feeds[a]) edge(0);  // the input chain delivers its spikes
         }
-    }
     chain_deps.assign(nc, {});
     int fuse = kMaxFuse;
     for (int a = 0; a < nc; ++a)
@@ -1345,16 +1389,13 @@ int eb_inject_spikes(eb_ctx *ctx, int64_t n, const float *time_s, const int64_t 
     };
     ctx->pending.reserve(ctx->pending.size() + (size_t)n);
     bool sorted = true;  // lists come in time order as a rule
+    if (ctx->finalized)  // a model neuron may be an input source, too
+        for (int64_t i = 0; i < n; ++i)
+            if (int rc = ctx->feed_population(ctx->pop_of[cell[i]])) return rc;
     for (int64_t i = 0; i < n; ++i) {
         const PendingIn p{time_s[i], cell[i], ctx->pending_seq++};
         sorted = sorted && (ctx->pending.empty() || !earlier(p, ctx->pending.back()));
         ctx->pending.push_back(p);
-        // a model neuron used as an input source can deliver twice in one step
-        if (ctx->finalized && ctx->pops[ctx->pop_of[cell[i]]].kind != KIND_INPUT) {
-            for (auto &q : ctx->pops) q.dev.may_repeat = 1;
-            ctx->graphs_valid = false;
-            ctx->pops_dirty = true;
-        }
     }
     if (!sorted) std::stable_sort(ctx->pending.begin(), ctx->pending.end(), earlier);
     return EB_OK;

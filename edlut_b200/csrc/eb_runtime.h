@@ -76,6 +76,12 @@ struct eb_ctx {
     bool has_inputs = false;
     bool inputs_concurrent = false;  // input fan-out can overlap the neuron updates
     int input_threads = 32;
+    // [population] input spikes enter here: input layers, and model populations from the
+    // first spike injected into one of their neurons on
+    std::vector<uint8_t> feeds;
+    struct PairDelay { int64_t lo = INT64_MAX, hi = -1; };
+    std::vector<PairDelay> pair_delay;  // [source population][target population], 0.1 ms units
+    std::vector<int64_t> max_out;       // [population] most output synapses of a neuron
     // persistent multi-step kernel
     bool persistent = false;        // opt-in (eb_set_persistent): grid barriers cost more than launches here
     bool persist_ok = false;        // set at finalize
@@ -170,8 +176,10 @@ struct eb_ctx {
     int prof_collect();
     int build_graph(int K);
     CachedGraph *graph_for(int K);
-    void plan_chains(const std::vector<int64_t> &out_ptr, const std::vector<uint32_t> &out_tgt,
-                     const std::vector<uint16_t> &out_units);
+    void plan_inputs();
+    void plan_chains();
+    int ensure_chain_streams();
+    int feed_population(int q);
     void enqueue_chains(int K);
     int setup_persistent();
     int seed_generators();

@@ -1175,12 +1175,13 @@ int eb_ctx::run_async(int64_t n) {
 }
 
 int eb_ctx::sync() {
+    if (!status) { set_error("not finalized"); return EB_ERR_STATE; }
     CK(cudaStreamSynchronize(stream));
     if (profile) {
         int rc = prof_collect();
         if (rc) return rc;
     }
-    const uint32_t f = status ? status->flags : 0u;
+    const uint32_t f = status->flags;
     if (f) {
         CK(cudaMemset(net.flags, 0, sizeof(uint32_t)));
         status->flags = 0;

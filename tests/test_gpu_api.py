@@ -351,3 +351,18 @@ def test_output_files_match_the_reference_files(tmp_path):
         sim.write_spikes(of)
         assert open(of, "rb").read() == b""
         sim.close()
+
+
+def test_sync_before_finalize_is_refused():
+    from edlut_b200 import _lib
+    from edlut_b200.configs import LIF_C1
+    from edlut_b200.simulation import Simulation
+    sim = Simulation()
+    sim.add_population("LIFTimeDrivenModel", 3, params=LIF_C1)
+    with pytest.raises(_lib.EdlutError, match="not finalized"):
+        sim.sync()
+    sim.set_connectivity([0], [1], [1e-3], [0], [0.5], [1.0])
+    sim.finalize()
+    sim.run(5)
+    sim.sync()
+    sim.close()

@@ -179,39 +179,68 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 
-// The op's own memory pool on a device.  Each call takes its scratch from it on the
-// caller's stream and gives it back there, so calls on different streams and threads
-// never share a block, and the pool keeps up to kPoolKept bytes of returned blocks when
-// the device synchronises: the default pool keeps none unless the process set it so,
-// and every call after a synchronisation mapped its scratch anew (100,000 arrivals,
-// waited for: 510-690 us, 90 with this pool).  Above kPoolKept everything goes back.
+// Id of the calling thread's current context, never that of an earlier one; 0 where the
+// driver does not tell.  What is kept per device below belongs to a context: it dies with
+// it in cudaDeviceReset, and its handle or address must not be used after that.
+unsigned long long context_id() {
+    using Fn = int (*)(void *, unsigned long long *);  // cuCtxGetId: (CUcontext, id), 0 on success
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? (Fn)p : nullptr;
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == 0 ? id : 0;
+}
+
+// The op's own memory pool on the current device, null where the device's current pool
+// serves instead.  Each call takes its scratch from it on the caller's stream and gives it
+// back there, so calls on different streams and threads never share a block, and the pool
+// keeps up to kPoolKept bytes of returned blocks when the device synchronises: the default
+// pool keeps none unless the process set it so, and every call after a synchronisation
+// mapped its scratch anew (100,000 arrivals, waited for: 480-530 us, 48 with this pool).
+// Above kPoolKept everything goes back.  A pool that the process set with
+// cudaDeviceSetMemPool is used as before, and so is the default one in any context but
+// the first that called on the device (after a reset of it, say).
 constexpr uint64_t kPoolKept = 32ull << 20;
 
-int fold_pool(cudaMemPool_t *out) {
+cudaMemPool_t fold_pool() {
+    struct Own {
+        cudaMemPool_t pool;
+        unsigned long long ctx;  // that of the first call, 0 before
+    };
     static std::mutex mu;
-    static cudaMemPool_t pools[kMaxDevices] = {};
+    static Own own[kMaxDevices] = {};
     int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) { set_error("cudaGetDevice: %s", cudaGetErrorString(e)); return EB_ERR_CUDA; }
-    if (dev < 0 || dev >= kMaxDevices) { set_error("device index %d above %d", dev, kMaxDevices - 1); return EB_ERR_ARG; }
+    cudaMemPool_t now = nullptr, standard = nullptr;
+    const unsigned long long ctx = context_id();
+    if (!ctx || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices ||
+        cudaDeviceGetMemPool(&now, dev) != cudaSuccess || cudaDeviceGetDefaultMemPool(&standard, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (now != standard) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
-    if (!pools[dev]) {
+    Own &o = own[dev];
+    if (!o.ctx) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
-        cudaMemPool_t p = nullptr;
         uint64_t kept = kPoolKept;
-        e = cudaMemPoolCreate(&p, &props);
-        if (e == cudaSuccess) {
-            e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &kept);
-            if (e != cudaSuccess) cudaMemPoolDestroy(p);
+        cudaMemPool_t p = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&p, &props);
+        if (e == cudaSuccess && (e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &kept)) != cudaSuccess)
+            cudaMemPoolDestroy(p);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
         }
-        if (e != cudaSuccess) { set_error("fold scratch pool on device %d: %s", dev, cudaGetErrorString(e)); return EB_ERR_CUDA; }
-        pools[dev] = p;
+        o = Own{p, ctx};
     }
-    *out = pools[dev];
-    return EB_OK;
+    return o.ctx == ctx ? o.pool : nullptr;
 }
 
 }  // namespace
@@ -228,12 +257,9 @@ extern "C" int eb_fold_arrivals(void *stream, int64_t n, const int32_t *target, 
     // under stream capture the scratch is a node of the graph, which owns it
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(st, &capture);
-    cudaMemPool_t pool = nullptr;
-    if (e == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
-        if ((rc = fold_pool(&pool))) return rc;
-        e = cudaMallocFromPoolAsync(&scratch, bytes, pool, st);
-    } else if (e == cudaSuccess) {
-        e = cudaMallocAsync(&scratch, bytes, st);
+    if (e == cudaSuccess) {
+        const cudaMemPool_t pool = capture == cudaStreamCaptureStatusNone ? fold_pool() : nullptr;
+        e = pool ? cudaMallocFromPoolAsync(&scratch, bytes, pool, st) : cudaMallocAsync(&scratch, bytes, st);
     }
     if (e != cudaSuccess) { set_error("fold scratch (%zu bytes): %s", bytes, cudaGetErrorString(e)); return EB_ERR_NOMEM; }
     rc = fold_enqueue(st, scratch, n, target, type, weight, time, n_targets, g_exc, g_inh, g_nmda);
@@ -263,19 +289,21 @@ constexpr size_t kNoAllocScratchBytes =
 
 static __device__ __align__(256) unsigned char g_fold_scratch[kNoAllocScratchBytes];
 
-// The array's device address on each device, looked up once per device (with
-// that device current); in host code g_fold_scratch only names a host-side
-// stand-in, never the device memory.
+// The array's device address on each device, looked up once per device and
+// context (with that device current); in host code g_fold_scratch only names a
+// host-side stand-in, never the device memory.
 std::mutex g_scratch_mu;
 void *g_scratch_ptr[kMaxDevices] = {};
+unsigned long long g_scratch_ctx[kMaxDevices] = {};
 
 int scratch_for_current_device(void **out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) { set_error("cudaGetDevice: %s", cudaGetErrorString(e)); return EB_ERR_CUDA; }
     if (dev < 0 || dev >= kMaxDevices) { set_error("device index %d above %d", dev, kMaxDevices - 1); return EB_ERR_ARG; }
+    const unsigned long long ctx = context_id();
     std::lock_guard<std::mutex> lock(g_scratch_mu);
-    if (!g_scratch_ptr[dev]) {
+    if (!g_scratch_ptr[dev] || !ctx || g_scratch_ctx[dev] != ctx) {
         void *p = nullptr;
         e = cudaGetSymbolAddress(&p, g_fold_scratch);
         if (e != cudaSuccess || !p) {
@@ -283,6 +311,7 @@ int scratch_for_current_device(void **out) {
             return EB_ERR_CUDA;
         }
         g_scratch_ptr[dev] = p;
+        g_scratch_ctx[dev] = context_id();
     }
     *out = g_scratch_ptr[dev];
     return EB_OK;

@@ -20,7 +20,6 @@ constexpr int kSweepWindow = 8;     // steps between meetings of a network's CTA
 constexpr int kRoundSources = 8;    // sources of a delivery batch from which it goes in rounds
 constexpr int kBidSlots = 1024;     // slots the rounds' entries bid for (a power of two)
 constexpr uint32_t kNoBid = 0xffffffffu;
-constexpr int64_t kDrainAtOnce = 1 << 20;  // spikes a drain copies without asking for their number first
 constexpr int kOwnObs = 1024;       // most observed neurons a network's threads record themselves
 constexpr int kTileMin = 256;       // fewest neurons a CTA of several per network is given
 constexpr int kBatch = 4;           // synapses per thread per delivery batch
@@ -186,12 +185,13 @@ struct eb_sweep {
     bool obs_slot_ok = false;           // obs_slot is that of the observed neurons set last
     double *red_out = nullptr;          // [n_nets][4] parameter gradient sums
     int64_t traj_steps = 0;
-    void *pin = nullptr;                // spike read-back (pinned)
-    size_t pin_bytes = 0;
+    std::vector<uint32_t> counts;       // spikes of every network so far
+    bool counts_ok = false;             // counts are those of the device (cleared by every launch that moves them)
+    std::vector<int32_t> ends;          // spike read-back
+    std::vector<uint16_t> cells;
     ~eb_sweep() {
         if (graph) cudaGraphExecDestroy(graph);
         for (void *p : allocs) cudaFree(p);
-        if (pin) cudaFreeHost(pin);
         if (stream) cudaStreamDestroy(stream);
     }
     int dalloc(void **p, size_t b) {

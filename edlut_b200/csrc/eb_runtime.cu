@@ -1388,7 +1388,9 @@ int eb_inject_spikes(eb_ctx *ctx, int64_t n, const float *time_s, const int64_t 
         if (a.t != b.t) return a.t < b.t;
         return a.seq < b.seq;
     };
-    ctx->pending.reserve(ctx->pending.size() + (size_t)n);
+    // (geometric: a reserve of the exact size would copy the backlog on every call)
+    const size_t want = ctx->pending.size() + (size_t)n;
+    if (want > ctx->pending.capacity()) ctx->pending.reserve(std::max(want, 2 * ctx->pending.capacity()));
     bool sorted = true;  // lists come in time order as a rule
     if (ctx->finalized)  // a model neuron may be an input source, too
         for (int64_t i = 0; i < n; ++i)

@@ -366,3 +366,21 @@ def test_sync_before_finalize_is_refused():
     sim.run(5)
     sim.sync()
     sim.close()
+
+
+def test_many_small_injections_cost_the_same_each():
+    """A call that queues one spike does not copy the spikes queued before it."""
+    import time
+    from edlut_b200.configs import LIF_C1
+    from edlut_b200.simulation import Simulation
+    sim = Simulation()
+    sim.add_population("LIFTimeDrivenModel", 3, params=LIF_C1)
+    took = []
+    for block in range(16):
+        t0 = time.perf_counter()
+        for k in range(5000):
+            sim.inject_spikes([1e-5 * (5000 * block + k)], [0])
+        took.append(time.perf_counter() - t0)
+    sim.close()
+    # copying the backlog made the last blocks some 15 times as long as the first
+    assert min(took[-4:]) < 4 * min(took[:4]), took

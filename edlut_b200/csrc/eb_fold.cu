@@ -33,15 +33,23 @@ __device__ __forceinline__ bool fold_less(const FoldRec &a, const FoldRec &b) {
     return a.t < b.t || (a.t == b.t && a.i < b.i);
 }
 
-// Arrivals of one target as a linked list: head[t] is its last linked arrival, next[i]
-// the one linked before arrival i (kNone: none).  The order of the links is whatever the
-// atomics give; the fold sorts.
+// Arrivals of one target as a linked list: the last linked arrival (kNone: none) and how
+// many more there are, less one (most targets' only arrival takes one atomic); next[i] is
+// the arrival linked before arrival i.  The order of the links is whatever the atomics
+// give; the fold sorts.
 constexpr uint32_t kNone = 0xffffffffu;
+struct alignas(8) FoldList {
+    uint32_t last, more;
+};
 
-__global__ void __launch_bounds__(256) k_fold_link(int64_t n, const int32_t *__restrict__ target, uint32_t *head,
+__global__ void __launch_bounds__(256) k_fold_link(int64_t n, const int32_t *__restrict__ target, FoldList *list,
                                                    uint32_t *__restrict__ next) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        next[i] = atomicExch(head + target[i], (uint32_t)i);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        FoldList *l = list + target[i];
+        const uint32_t before = atomicExch(&l->last, (uint32_t)i);
+        next[i] = before;
+        if (before != kNone) atomicAdd(&l->more, 1u);
+    }
 }
 
 // Restore the heap property below node j of the max-heap r[0..c) by (time, index).
@@ -83,82 +91,151 @@ __device__ __forceinline__ void fold_sort(FoldRec *r, uint32_t c) {
     }
 }
 
-// One thread per target: walk its list, keep the arrivals sorted by (time, index), then
-// add the weights in that order.  Bound by the walk's dependent loads, so everything an
-// arrival needs is loaded as it is met.  More than kFoldLocal arrivals are gathered into
-// `rec` (a run of it taken with `used`, which starts one below zero) and sorted there.
-constexpr uint32_t kFoldLocal = 16;
+// The same by a warp, in place: a bitonic sort whose every comparison moves the smaller
+// record down (the first of each merge compares mirrored places), so that the places
+// beyond c may be left out.
+__device__ __forceinline__ void fold_sort_warp(FoldRec *r, uint64_t c, int lane) {
+    auto order = [&](uint64_t i, uint64_t j) {
+        const FoldRec x = r[i], y = r[j];
+        if (fold_less(y, x)) { r[i] = y; r[j] = x; }
+    };
+    for (uint64_t k = 2; k < 2 * c; k <<= 1) {
+        for (uint64_t p = lane;; p += 32) {
+            const uint64_t lo = p / (k / 2) * k, o = p % (k / 2);
+            if (lo + k / 2 >= c) break;  // no pair of this merge or a later one
+            if (lo + k - 1 - o < c) order(lo + o, lo + k - 1 - o);
+        }
+        __syncwarp();
+        for (uint64_t s = k / 4; s > 0; s >>= 1) {
+            for (uint64_t p = lane;; p += 32) {
+                const uint64_t i = p / s * 2 * s + p % s;
+                if (i + s >= c) break;
+                order(i, i + s);
+            }
+            __syncwarp();
+        }
+    }
+}
 
-__global__ void __launch_bounds__(128) k_fold_apply(int64_t m, const uint32_t *__restrict__ head, const uint32_t *__restrict__ next,
-                                                    const double *__restrict__ time, const int8_t *__restrict__ type,
-                                                    const float *__restrict__ weight, uint32_t *used, FoldRec *rec,
-                                                    float *g_exc, float *g_inh, float *g_nmda) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    const uint32_t i = head[t];
-    if (i == kNone) return;
-    float ge = g_exc ? g_exc[t] : 0.0f, gi = g_inh ? g_inh[t] : 0.0f, gn = g_nmda ? g_nmda[t] : 0.0f;
+// One thread per target: walk its list, keep the arrivals sorted by (time, index), then
+// add the weights in that order.  Bound by the walk's dependent loads (0.7 us an arrival),
+// so everything an arrival needs is loaded as it is met.  More than kFoldLocal arrivals are
+// gathered into `rec` (a run of it taken with `used`, which starts one below zero) and
+// sorted there: by the thread, or beyond kFoldThread by the whole warp, one such list after
+// the other, unless the warp has more than kFoldLong of them to sort at once.  100,000
+// arrivals at 30,000 targets: 29 us; with 1,000 of them at each of four targets 0.44 ms
+// (thread's sort of counted and scattered records 1.6, of a list walked three times 4.1);
+// 10,000 at 8 targets 0.52 ms (6.3, 7.0).
+constexpr uint32_t kFoldLocal = 16, kFoldThread = 96;
+constexpr int kFoldLong = 12;
+
+__global__ void __launch_bounds__(128) k_fold_apply(int64_t m, const FoldList *__restrict__ list, const uint32_t *__restrict__ next, const double *__restrict__ time,
+                                                    const int8_t *__restrict__ type, const float *__restrict__ weight,
+                                                    uint32_t *used, FoldRec *rec, float *g_exc, float *g_inh, float *g_nmda,
+                                                    int per_warp) {
+    constexpr unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t t = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane;
+    const FoldList own = lane < per_warp && t < m ? list[t] : FoldList{kNone, kNone};
+    const uint32_t c = own.last == kNone ? 0u : own.more + 2u;
+    if (!__any_sync(full, c != 0)) return;
+    float ge = 0.0f, gi = 0.0f, gn = 0.0f;
+    if (c) {
+        ge = g_exc ? g_exc[t] : 0.0f;
+        gi = g_inh ? g_inh[t] : 0.0f;
+        gn = g_nmda ? g_nmda[t] : 0.0f;
+    }
     auto add = [&](int ty, float w) {
         if (ty == 0) ge += w;
         else if (ty == 1) gi += w;
         else gn += w;
     };
-    FoldRec key[kFoldLocal];
-    float w[kFoldLocal];
-    int8_t ty[kFoldLocal];
-    uint32_t c = 0;
-    uint32_t rest = i;
-    for (; rest != kNone && c < kFoldLocal; ++c) {
-        const FoldRec v{time ? time[rest] : 0.0, rest, 0};
-        const float vw = weight[rest];
-        const int8_t vt = type[rest];
-        rest = next[rest];
-        int b = (int)c - 1;
-        while (b >= 0 && fold_less(v, key[b])) {
-            key[b + 1] = key[b];
-            w[b + 1] = w[b];
-            ty[b + 1] = ty[b];
-            --b;
-        }
-        key[b + 1] = v;
-        w[b + 1] = vw;
-        ty[b + 1] = vt;
-    }
-    if (rest == kNone) {
-        for (uint32_t a = 0; a < c; ++a) add(ty[a], w[a]);
-    } else {
-        for (uint32_t q = rest; q != kNone; q = next[q]) ++c;
-        FoldRec *r = rec + (atomicAdd(used, c) + 1u);
+    FoldRec *r = nullptr;
+    if (c > kFoldLocal) {
+        r = rec + (atomicAdd(used, c) + 1u);
         uint32_t a = 0;
-        for (uint32_t q = i; q != kNone; q = next[q]) r[a++] = FoldRec{time ? time[q] : 0.0, q, 0};
-        fold_sort(r, c);
-        for (a = 0; a < c; ++a) add(type[r[a].i], weight[r[a].i]);
+        for (uint32_t q = own.last; q != kNone; q = next[q]) r[a++] = FoldRec{time ? time[q] : 0.0, q, 0};
+    } else if (c) {
+        FoldRec key[kFoldLocal];
+        float w[kFoldLocal];
+        int8_t ty[kFoldLocal];
+        uint32_t q = own.last;
+        for (uint32_t a = 0; a < c; ++a) {
+            const FoldRec v{time ? time[q] : 0.0, q, 0};
+            const float vw = weight[q];
+            const int8_t vt = type[q];
+            q = next[q];
+            int b = (int)a - 1;
+            while (b >= 0 && fold_less(v, key[b])) {
+                key[b + 1] = key[b];
+                w[b + 1] = w[b];
+                ty[b + 1] = ty[b];
+                --b;
+            }
+            key[b + 1] = v;
+            w[b + 1] = vw;
+            ty[b + 1] = vt;
+        }
+        for (uint32_t a = 0; a < c; ++a) add(ty[a], w[a]);
     }
-    if (g_exc) g_exc[t] = ge;
-    if (g_inh) g_inh[t] = gi;
-    if (g_nmda) g_nmda[t] = gn;
+    unsigned longer = __ballot_sync(full, c > kFoldThread);
+    if (__popc(longer) > kFoldLong) longer = 0;
+    if (c > kFoldLocal && !(longer >> lane & 1)) {
+        fold_sort(r, c);
+        for (uint32_t a = 0; a < c; ++a) add(type[r[a].i], weight[r[a].i]);
+    }
+    for (; longer; longer &= longer - 1u) {
+        const int l = __ffs(longer) - 1;
+        FoldRec *rl = (FoldRec *)__shfl_sync(full, (unsigned long long)r, l);
+        const uint32_t cl = __shfl_sync(full, c, l);
+        __syncwarp();  // the owner's records are written
+        fold_sort_warp(rl, cl, lane);
+        for (uint32_t a0 = 0; a0 < cl; a0 += 32) {  // 32 loaded at once, added by the owner in order
+            const uint32_t k = min(32u, cl - a0);
+            int vt = 0;
+            float vw = 0.0f;
+            if (lane < k) {
+                const uint32_t i = rl[a0 + lane].i;
+                vt = type[i];
+                vw = weight[i];
+            }
+            for (uint32_t u = 0; u < k; ++u) {
+                const int tu = __shfl_sync(full, vt, u);
+                const float wu = __shfl_sync(full, vw, u);
+                if (lane == l) add(tu, wu);
+            }
+        }
+    }
+    if (c) {
+        if (g_exc) g_exc[t] = ge;
+        if (g_inh) g_inh[t] = gi;
+        if (g_nmda) g_nmda[t] = gn;
+    }
 }
 
-// Scratch layout shared by the entry points: heads (m) and the count of records taken,
-// links (n), then the records (16-byte aligned).
-size_t fold_words(int64_t n, int64_t m) { return (size_t)(m + 1) + (size_t)n; }
+// Scratch layout shared by the entry points: lists (m), the count of records taken, links
+// (n), then the records (16-byte aligned).
+constexpr size_t fold_words(int64_t n, int64_t m) { return 2 * (size_t)m + 1 + (size_t)n; }
 
-size_t fold_scratch_bytes(int64_t n, int64_t m) {
+constexpr size_t fold_scratch_bytes(int64_t n, int64_t m) {
     return ((fold_words(n, m) * sizeof(uint32_t) + 255) & ~(size_t)255) + (size_t)n * sizeof(FoldRec);
 }
 
 // Three launches (clear, link, fold); counting, scanning and scattering the arrivals
-// instead took eight.  100,000 arrivals at 30,000 targets: 34 us a
-// call among others with the copies of three conductance arrays, 57 before.
+// instead took eight (100,000 arrivals at 30,000 targets: 97 us a call among others, 29).
 int fold_enqueue(cudaStream_t st, void *scratch, int64_t n, const int32_t *target, const int8_t *type,
                  const float *weight, const double *time, int64_t m, float *g_exc, float *g_inh, float *g_nmda) {
     if (n == 0) return EB_OK;
-    uint32_t *head = (uint32_t *)scratch, *used = head + m, *next = head + m + 1;
+    FoldList *list = (FoldList *)scratch;
+    uint32_t *used = (uint32_t *)(list + m), *next = used + 1;
     FoldRec *rec = (FoldRec *)((char *)scratch + ((fold_words(n, m) * sizeof(uint32_t) + 255) & ~(size_t)255));
-    cudaError_t e = cudaMemsetAsync(head, 0xff, sizeof(uint32_t) * (size_t)(m + 1), st);  // no arrivals, no records
+    cudaError_t e = cudaMemsetAsync(list, 0xff, sizeof(uint32_t) * (size_t)(2 * m + 1), st);  // no arrivals, no records
     if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return EB_ERR_CUDA; }
-    k_fold_link<<<(int)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, st>>>(n, target, head, next);
-    k_fold_apply<<<(int)((m + 127) / 128), 128, 0, st>>>(m, head, next, time, type, weight, used, rec, g_exc, g_inh, g_nmda);
+    k_fold_link<<<(int)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, st>>>(n, target, list, next);
+    // few targets take a warp each, or a few a warp, until every SM sub-partition has one
+    const int per_warp = (int)std::min<int64_t>(32, (m + 148 * 4 - 1) / (148 * 4));
+    k_fold_apply<<<(int)((m + 4 * per_warp - 1) / (4 * per_warp)), 128, 0, st>>>(m, list, next, time, type, weight, used, rec, g_exc, g_inh,
+                                                                                g_nmda, per_warp);
     e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("fold kernels: %s", cudaGetErrorString(e)); return EB_ERR_CUDA; }
     return EB_OK;
@@ -273,7 +350,7 @@ extern "C" int eb_fold_arrivals(void *stream, int64_t n, const int32_t *target, 
 // or a host engine that claims all device memory for itself at start-up.  This
 // form of the op takes its scratch from a fixed array in the library's device
 // image instead.  Every GPU that loads the library holds that array (about
-// 6 MiB) until the process exits; it bounds one call to kNoAllocMaxArrivals
+// 7 MiB) until the process exits; it bounds one call to kNoAllocMaxArrivals
 // arrivals and kNoAllocMaxTargets targets.  All calls share the one array and
 // it keeps the previous call's contents: the counters that must start clear
 // are cleared at the start of every call, and two calls whose work overlaps on
@@ -283,9 +360,7 @@ namespace {
 
 constexpr int64_t kNoAllocMaxArrivals = 1 << 18;
 constexpr int64_t kNoAllocMaxTargets = 1 << 18;
-constexpr size_t kNoAllocScratchBytes =
-    (((size_t)(kNoAllocMaxTargets + 1 + kNoAllocMaxArrivals) * sizeof(uint32_t) + 255) & ~(size_t)255) +
-    (size_t)kNoAllocMaxArrivals * sizeof(FoldRec);
+constexpr size_t kNoAllocScratchBytes = fold_scratch_bytes(kNoAllocMaxArrivals, kNoAllocMaxTargets);
 
 static __device__ __align__(256) unsigned char g_fold_scratch[kNoAllocScratchBytes];
 

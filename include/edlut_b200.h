@@ -273,7 +273,7 @@ int eb_fold_arrivals(void *stream, int64_t n, const int32_t *target, const int8_
  * memory while they run (a closed-loop real-time controller whose step deadline
  * must not contain allocator calls, or a host engine that claims all device memory
  * at start-up).  No counterpart in the reference.  Its scratch is a fixed array in
- * the library's device image (about 6 MiB, held on every GPU that loads the library
+ * the library's device image (about 7 MiB, held on every GPU that loads the library
  * until exit), so one call takes at most 262144 arrivals and 262144 targets; larger
  * batches return EB_ERR_ARG.  It runs on the calling thread's current device; the
  * first call on a device looks up that array's address (cudaGetSymbolAddress) and

@@ -1573,7 +1573,6 @@ int eb_sweep_set_observed(eb_sweep *h, int m, const int32_t *idx) {
     }
     h->G.n_obs = m;
     h->obs_slot_ok = false;
-    h->h_obs.assign(idx, idx + (size_t)h->n_nets * m);
     if (h->graph) {
         cudaGraphExecDestroy(h->graph);
         h->graph = nullptr;

@@ -174,7 +174,6 @@ struct eb_sweep {
     // observation and checkpoints
     int ckpt_every = 0, n_ckpt = 0;
     int64_t ckpt_upto = -1;             // a checkpointed run from step 0 has reached this step
-    std::vector<int32_t> h_obs;         // observed neurons [n_nets][n_obs]
     std::vector<void *> ckpt;           // per slot: one block holding every state array
     // adjoint scratch (allocated on first use)
     float *lamV = nullptr, *lamE = nullptr, *lamI = nullptr;

@@ -1212,13 +1212,13 @@ int eb_sweep_configure(eb_sweep *h, int block, int steps_per_launch) {
     if (nb != 128 && nb != 256 && nb != 512 && nb != 1024) { set_error("block must be 128, 256, 512 or 1024"); return EB_ERR_ARG; }
     if (steps_per_launch < 0) { set_error("steps_per_launch < 0"); return EB_ERR_ARG; }
     const size_t smem = smem_of(ctas, cap);
-    // the largest any sweep of the process needs: another handle may have raised it
+    // The attribute belongs to the kernel, not to the handle: every handle sets the most
+    // there is, so that none takes away what another one's launches need, in whatever order
+    // their threads come here.
     for (bool traj : {false, true}) {
-        const void *f = (const void *)sweep_fn(h->integ, traj, ctas > 1);
-        cudaFuncAttributes fa;
-        SK(cudaFuncGetAttributes(&fa, f));
-        if ((size_t)fa.maxDynamicSharedSizeBytes >= smem) continue;
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = smem > room ? cudaErrorInvalidValue
+                                          : cudaFuncSetAttribute((const void *)sweep_fn(h->integ, traj, ctas > 1),
+                                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
         if (e != cudaSuccess) {
             cudaGetLastError();
             set_error("sweep kernel: %zu bytes of shared memory unavailable (%s)", smem, cudaGetErrorString(e));

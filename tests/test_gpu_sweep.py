@@ -244,3 +244,24 @@ def test_first_read_back_of_a_new_handle_costs_what_the_later_ones_do():
         sw.close()
         best = min(best, took[0] - min(took[1:]))
     assert best < 2e-3, best
+
+
+def test_sweeps_configured_by_several_threads_at_once():
+    # large and small sweeps share the kernel whose shared memory each of them needs
+    from concurrent.futures import ThreadPoolExecutor
+    nsteps = 20
+    specs = {n: sweep_networks(seed=n, n_networks=80, n_min=n, n_max=n + 50, t_end=nsteps * 1e-4, p=0.002)
+             for n in (3000, 100)}
+
+    def work(n):
+        for _ in range(6):
+            sw = make_sweep(specs[n], nsteps)
+            for _ in range(3):
+                sw.configure()
+                sw.reset()
+                sw.run(nsteps)
+            sw.close()
+        return True
+
+    with ThreadPoolExecutor(4) as pool:
+        assert all(pool.map(work, (3000, 100, 3000, 100)))

@@ -60,3 +60,53 @@ def test_burst_sizes_match_oracle(model, integrator, n, burst, plastic):
     assert sorted(zip(st.tolist(), ce.tolist())) == sorted(zip(o["spike_step"].tolist(), o["spike_cell"].tolist()))
     np.testing.assert_array_equal(trace, o["trace"].astype(np.float32))
     np.testing.assert_array_equal(w, o["w_final"].astype(np.float32))
+
+
+# Arrivals of one step at each neuron, around the 255 from which a lane's packed count is
+# read again; all at one delay, so that they come in the same step.
+SATURATED = (254, 255, 256, 300, 17, 1, 0, 511)
+
+
+def saturated_network(model, integrator, plastic, dt=1e-4):
+    from edlut_b200.network import Layer, NetworkDescription
+    rng = np.random.default_rng(len(model))
+    net = NetworkDescription()
+    inp = net.add_layer(Layer(max(SATURATED), "InputSpikeNeuronModel", output=0))
+    pop = net.add_layer(Layer(len(SATURATED), model, {}, integrator=integrator, dt=dt, name="pop"))
+    net.rules.append(("STDP", [0.004, 0.02, 0.0042, 0.02]))
+    src = np.concatenate([rng.choice(max(SATURATED), k, replace=False) for k in SATURATED])
+    tgt = np.repeat(np.asarray(pop), SATURATED)
+    net.add_synapses(src + inp.start, tgt, 1e-3, (src % 3 == 2).astype(np.int32), (rng.random(len(src)) * 0.15).astype(np.float32),
+                     0.3, 0 if plastic else -1)
+    net.add_synapses(np.asarray(pop), np.roll(pop, 1), 1e-3, 0, np.float32(0.5), np.float32(1.0), 0 if plastic else -1)
+    steps = (5, 21, 22, 47)  # a burst alone, two in consecutive steps, one late in a window
+    t = np.concatenate([(s + 0.1 + 0.5 * np.sort(rng.random(max(SATURATED)))) * dt for s in steps]).astype(np.float32)
+    c = np.concatenate([rng.permutation(max(SATURATED)) for _ in steps]) + inp.start
+    # the counts meant: every input fires once a burst, one delay, all inside one step
+    grid = np.concatenate([[0.0], np.cumsum(np.full(100, float(np.float32(dt))))])
+    arrival = np.searchsorted(grid, t.astype(np.float64) + 10 * 0.0001, side="right")
+    for j, k in enumerate(SATURATED):
+        own = np.bincount(arrival[np.isin(c - inp.start, src[tgt == pop.start + j])], minlength=100) if k else np.zeros(100, int)
+        assert own.max() == k and (own == k).sum() == (len(steps) if k else 100)
+    return net, t, c
+
+
+@pytest.mark.parametrize("plastic", [True, False])
+@pytest.mark.parametrize("model,integrator", [("LIFTimeDrivenModel", "Euler"), ("AdExTimeDrivenModel", "RK2"), ("HHTimeDrivenModel", "BDF")])
+def test_counts_beyond_the_packed_byte_match_oracle(model, integrator, plastic):
+    from edlut_b200.simulation import Simulation
+    from oracle import oracle as O
+    net, t, c = saturated_network(model, integrator, plastic)
+    first, n, steps = net.layers[0].n, len(SATURATED), 80
+    o = O.run(net, t, c, steps, trace=(steps, first, n))
+    sim = Simulation.from_description(net)
+    sim.inject_spikes(t, c)
+    sim.set_trace(first, n, steps)
+    sim.run(steps)
+    st, ce = sim.spikes()
+    trace, w, events = sim.get_trace(), sim.weights(), sim.counters()["events"]
+    sim.close()
+    assert sorted(zip(st.tolist(), ce.tolist())) == sorted(zip(o["spike_step"].tolist(), o["spike_cell"].tolist()))
+    np.testing.assert_array_equal(trace, o["trace"].astype(np.float32))
+    np.testing.assert_array_equal(w, o["w_final"].astype(np.float32))
+    assert events == o["n_events"]

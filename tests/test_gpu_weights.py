@@ -26,3 +26,22 @@ def test_weights_keep_file_order(m):
     sim.set_weights(new if m else np.zeros(1, np.float32))
     np.testing.assert_array_equal(sim.weights(), new)
     sim.close()
+
+
+def test_weights_of_more_than_one_staging_pass():
+    """More synapses than the staging buffer holds (8 << 20): the second pass takes the rest."""
+    from edlut_b200.network import Layer, NetworkDescription
+    from edlut_b200.simulation import Simulation
+    m = (8 << 20) + 257
+    rng = np.random.default_rng(1)
+    net = NetworkDescription()
+    net.add_layer(Layer(2000, "InputSpikeNeuronModel", output=0))
+    net.add_layer(Layer(9000, "LIFTimeDrivenModel", {}, integrator="Euler"))
+    w = rng.random(m, dtype=np.float32)
+    net.add_synapses(rng.integers(0, 2000, m), 2000 + rng.integers(0, 9000, m), 1e-3, 0, w, np.float32(2.0), -1)
+    sim = Simulation.from_description(net)
+    np.testing.assert_array_equal(sim.weights(), w)
+    new = rng.random(m, dtype=np.float32)
+    sim.set_weights(new)
+    np.testing.assert_array_equal(sim.weights(), new)
+    sim.close()
